@@ -1,6 +1,9 @@
 // ATM three-body kernel, precision form: the per-visit triplet arithmetic in FP32.
-// Same enumeration, schedule, weights and mirror-symmetric accumulation as k_atm
-// (d3_atm.cuh); per-entry set-up (C6 of the apex pairs, damping ratios) is done in FP64
+// Same enumeration and weights as k_atm64 (d3_atm.cuh). Each thread owns one list entry x
+// (handed out in order of distance from the apex, so the lanes of a warp have similar
+// numbers of partners in range) and visits every partner y of a staged tile that passes
+// its distance test; every unordered pair is visited from both of its entries and all
+// accumulation into x is thread-private. Per-entry set-up (C6 of the apex pairs, damping ratios) is done in FP64
 // and rounded once. Per-visit sums, dE/dCN included, are kept in FP32 within one
 // partner tile and carried across tiles in FP64 (blocked summation, error
 // ~ sqrt(tile) * eps_32 per block).
@@ -10,6 +13,9 @@
 // 32-bit in-range masks over tiles padded to a multiple of 32 with far-away dummies.
 
 constexpr int ATM32_NRP = 8; // padded C6 row length (NR <= 7)
+constexpr int ATM_THREADS = 128;
+constexpr int ATM_PERM_CAP = 8192; // longest list whose entries are re-ordered by distance
+constexpr int ATM_SHELLS = 32;
 
 template <int NR, bool CENTER>
 __global__ void __launch_bounds__(ATM_THREADS) k_atm32(KP p, int tile) {

@@ -1199,6 +1199,7 @@ struct Engine {
     DBuf<float4> xs32;
     DBuf<float> w32, dw32, Y32, YD32;
     DBuf<float4> atmb_scratch;
+    DBuf<Atm64Row> atm64_scratch;
     DBuf<long long> atm_off;
     DBuf<int2> atm_ent;
     long long atm_cap = 0;
@@ -1223,7 +1224,7 @@ struct Engine {
         const void *fn = nullptr;
         size_t sm = 0;
         int blocks = 1;
-    } atm_occ_cache[12]; // 0-3 mirror / FP64 ATM, 5 grouped two-body, 8-11 block-pair ATM
+    } atm_occ_cache[12]; // 0, 2, 4 FP64 ATM, 1, 3 mirror, 5 grouped two-body, 8-11 block-pair ATM
     SurrState surr;
     int shard_rank = 0, shard_world = 0; // set by engine_shard_begin
 
@@ -1242,6 +1243,7 @@ struct Engine {
         Y32.release();
         YD32.release();
         atmb_scratch.release();
+        atm64_scratch.release();
         xw_in.release();
         xs.release();
         atm_off.release();
@@ -1809,6 +1811,27 @@ static int pairs_occupancy(Engine *e) {
     return c.blocks;
 }
 
+// CTAs per SM of the FP64 ATM kernel, their shared memory and the splits of an apex
+struct Atm64Shape {
+    int ctas, nrows, split;
+    size_t fixed, tile_bytes;
+};
+static Atm64Shape atm64_shape(const Engine *e, int world) {
+    Atm64Shape sh;
+    const int want = e->opt.atm_ctas_per_sm;
+    sh.ctas = want <= 0 ? 1 : (want >= 4 ? 4 : (want >= 2 ? 2 : 1));
+    sh.nrows = ATM64_ROWS / sh.ctas;
+    const size_t limit = std::min<size_t>(227 * 1024, 228 * 1024 / sh.ctas - 1024) - ATM64_STATIC;
+    sh.fixed = atm64_fixed_bytes(e->ne, e->nref, ATM64_THREADS / 32 / sh.ctas, sh.nrows);
+    sh.tile_bytes = limit - sh.fixed;
+    const long long apexes = std::max<long long>(1, (long long)e->n / std::max(1, world));
+    const long long items = 6LL * e->dev_sms * sh.ctas;
+    // about six items per CTA, so that systems of few apexes fill the GPU and the last items
+    // are short against the pass (16-atom cell 26.8 -> 0.5 ms, 96 atoms 36 -> 3.4 ms)
+    sh.split = (int)std::max<long long>(1, std::min<long long>(32, (items + apexes - 1) / apexes));
+    return sh;
+}
+
 static KP make_kp(Engine *e) {
     KP p;
     memset(&p, 0, sizeof(p));
@@ -1868,6 +1891,10 @@ static KP make_kp(Engine *e) {
         const int ctas = e->dev_sms * sh.ctas;
         p.atmb_split = e->opt.atmb_split > 0 ? std::min(e->opt.atmb_split, 64)
                                              : std::max(1, std::min(16, (3 * ctas + p.n - 1) / std::max(1, p.n)));
+    }
+    if (e->use_atm && !p.precision) {
+        const Atm64Shape sh = atm64_shape(e, 1);
+        e->atm64_scratch.ensure((size_t)e->dev_sms * sh.ctas * sh.nrows);
     }
     p.atm_force_scaled = e->opt.atm_force_scaled ? 1 : 0;
     p.anyshift = e->anyshift.p;
@@ -1958,6 +1985,32 @@ static void launch_blockpair(Engine *e, const KP &p, cudaStream_t s, const AtmbS
     atm_occupancy(e, 8 + (shb.nbuf == 2 ? 0 : 2) + (simple ? 1 : 0), smb, fn);
     void *args[] = {(void *)&p, (void *)&e->atmb_scratch.p};
     D3_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(32 * shb.warps), args, smb, s));
+}
+
+// FP64 ATM pass: one launch per apex kind present (weight-free structures, the others), or
+// the centre mode of the surrogate fallback
+template <int NR>
+static void launch_atm64(Engine *e, const KP &p0, cudaStream_t s, bool center) {
+    KP p = p0;
+    const Atm64Shape sh = atm64_shape(e, p.shard_world);
+    p.atmb_split = sh.split;
+    const size_t sm = sh.fixed + sh.tile_bytes;
+    const int tile_max = e->opt.atm_tile > 0 ? std::max(32, std::min(e->opt.atm_tile, 65504) & ~31) : 65504;
+    const int grid = e->dev_sms * sh.ctas;
+    bool kind[3] = {false, false, center};
+    if (!center)
+        for (const SG &q : e->sg) kind[q.atm_simple ? ATM64_SIMPLE : ATM64_WEIGHTED] = true;
+    const void *fns[3] = {(const void *)k_atm64<NR, ATM64_SIMPLE>, (const void *)k_atm64<NR, ATM64_WEIGHTED>,
+                          (const void *)k_atm64<NR, ATM64_CENTER>};
+    const int cache[3] = {0, 4, 2};
+    for (int k = 0; k < 3; ++k) {
+        if (!kind[k]) continue;
+        if (k == ATM64_WEIGHTED && kind[ATM64_SIMPLE]) D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
+        atm_occupancy(e, cache[k], sm, fns[k]);
+        int nrows = sh.nrows, tile_bytes = (int)sh.tile_bytes, tmax = tile_max;
+        void *args[] = {(void *)&p, (void *)&e->atm64_scratch.p, &nrows, &tile_bytes, &tmax};
+        D3_CUDA(cudaLaunchKernel(fns[k], dim3(grid), dim3(ATM64_THREADS / sh.ctas), args, sm, s));
+    }
 }
 
 static SurrDesc surr_desc(const int *chan, int nch, float *G, const float *dEdG, int *center) {
@@ -2130,21 +2183,7 @@ static void launch_all(Engine *e, const KP &p0, cudaStream_t s, int stage = 0, d
                 else
                     k_atm32<NR, false><<<grid, ATM_THREADS, sm, s>>>(pc, tile);
             } else {
-                // partner tile: as many entries as fit in ~160 KB next to the apex tables
-                const size_t fixed = (size_t)p.ne * NR * sizeof(double) + (size_t)p.ne * p.ne * sizeof(double) +
-                                     ATM_PERM_CAP * sizeof(unsigned short);
-                const size_t per = sizeof(Partner) + (size_t)p.ne * NR * sizeof(double);
-                const int tmax = (int)std::max<size_t>(8, std::min<size_t>(256, (160 * 1024 - fixed) / per));
-                const int tile = e->opt.atm_tile > 0 ? std::min(tmax, std::max(8, e->opt.atm_tile)) : std::min(tmax, 128);
-                const size_t sm = (size_t)tile * per + fixed;
-                const void *fn = surr ? (const void *)k_atm<NR, true> : (const void *)k_atm<NR, false>;
-                const int blocks_per_sm = atm_occupancy(e, surr ? 2 : 0, sm, fn);
-                const int per_sm = e->opt.atm_ctas_per_sm > 0 ? std::min(e->opt.atm_ctas_per_sm, blocks_per_sm) : blocks_per_sm;
-                const int grid = std::max(1, std::min(n, e->dev_sms * std::max(1, per_sm)));
-                if (surr)
-                    k_atm<NR, true><<<grid, ATM_THREADS, sm, s>>>(pc, tile);
-                else
-                    k_atm<NR, false><<<grid, ATM_THREADS, sm, s>>>(pc, tile);
+                launch_atm64<NR>(e, pc, s, surr);
             }
             if (surr) k_desc_bwd<NR><<<gw, T, 0, s>>>(p, sd);
         }
