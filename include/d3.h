@@ -135,8 +135,8 @@ enum {
                                     0 = as many as the shared memory allows (4,096..8,192);
                                     longer lists go to the mirror-symmetric kernel */
     D3_OPT_ATMB_SPLIT = 13,      /* CTAs of the block-pair kernel sharing one apex, each taking
-                                    every S-th block row (0 = automatic: more than one only
-                                    when the apexes are fewer than about 3 per CTA, e.g. the
+                                    every S-th block row (0 = automatic: the S that fills the
+                                    GPU's CTAs best when apexes are few, e.g. 3 for the
                                     96-atom water box; 1..64) */
     D3_OPT_ATMB_FINE_SKIP = 14   /* block-pair kernel: 1 (default) skips out-of-range visits
                                     per two steps, 0 per four steps (more overlap of the

@@ -1,20 +1,13 @@
 // ATM three-body kernel, FP64 (replaces the reference's atm_kernel, src/d3_kernel.cu:1199-1509).
 // Included by d3_engine.cu after the kernel parameter block and the shared helpers.
 //
-// Enumeration: for each apex a, the half list L_a = {(j, T): j <= a in caller order,
+// Enumeration: for each apex a, the half list L_a = {(j, T) before (a, 0) (atm_before):
 // 1e-12 <= r^2 <= rc_ATM^2} built by k_atm_list; a triplet is an unordered pair of
-// distinct entries {x, y} of L_a with 1e-12 <= r_xy^2 <= rc_ATM^2. This is the
-// reference's (b, T_b, c, T_c) loop with c <= b (src/d3_kernel.cu:1235-1327); its
-// repeated-index scale factors (:1282-1290) become a weight per unordered pair:
-//     distinct atoms, none equal to a     w = 1     (reference force weight 1)
-//     distinct atoms, one is a's image    w = 1/2   (force weight 1)
-//     same atom, not a                    w = 1     (force weight 2)
-//     same atom, equal to a               w = 1/3   (force weight 2)
-// (the reference applies the scale to energy, dE/dCN and stress but not to forces;
-// the force weight reproduces that, or equals w when atm_force_scaled is set).
+// distinct entries {x, y} of L_a with 1e-12 <= r_xy^2 <= rc_ATM^2. With the reference's
+// order (entries j <= a in caller order) this is its (b, T_b, c, T_c) loop with c <= b
+// (src/d3_kernel.cu:1235-1327). Repeated atoms change the weights (atm_weights).
 //
-// Schedule: persistent CTAs pull (apex, split) items from a work counter, largest lists
-// first; the splits of an apex share its entries x (rows) between CTAs, so that systems of
+// Schedule: persistent CTAs pull (apex, split) items from a work counter; the splits of an apex share its entries x (rows) between CTAs, so that systems of
 // few apexes fill the GPU. A warp owns one row x at a time. It tests x against the staged
 // partners 32 at a time (FP32 positions; pairs near a limit again in FP64) and queues the
 // ones in range; when 32 are queued, all 32 lanes visit one partner y each. Every visit
@@ -265,6 +258,7 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Row *scra
         const int a = KIND == ATM64_CENTER ? p.atm_apex[item] : p.sorted_of[p.n - 1 - item];
         const SG &g = p.sg[p.sid[a]];
         if (KIND != ATM64_CENTER && (g.atm_simple != 0) != (KIND == ATM64_SIMPLE)) continue; // the other instance's
+        const bool ref = KIND == ATM64_WEIGHTED && atm_reference_order(p, g, p.sid[a]);
         const long long e0 = p.atm_off[a];
         const int m = (int)(p.atm_off[a + 1] - e0);
         const double4 xa = p.xs[a];
@@ -431,14 +425,12 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Row *scra
                                 for (int h = 0; h < 2; ++h)
                                     atm64_visit<NR>(vx, vy, vz, d1, id1, h1, p1, g1, wx, dwx, sA + 3 * k[h], sRx + RQ * k[h], V[h]);
                                 if (KIND == ATM64_WEIGHTED) {
-                                    // reference scale factors (src/d3_kernel.cu:1282-1290)
                                     const int jy[2] = {__float_as_int(sF[k[0]].w), __float_as_int(sF[k[1]].w)};
                                     if (jx == jy[0] || jx == jy[1] || jx == a || jy[0] == a || jy[1] == a) {
 #pragma unroll
                                         for (int h = 0; h < 2; ++h) {
-                                            const bool same = jx == jy[h], own = jx == a || jy[h] == a;
-                                            const double w = same ? (own ? third : 1.0) : (own ? 0.5 : 1.0);
-                                            const double wf = p.atm_force_scaled ? w : (same ? 2.0 : 1.0);
+                                            double w, wf;
+                                            atm_weights(jx == jy[h], jx == a, jy[h] == a, ref, p.atm_force_scaled != 0, w, wf);
                                             const double d3w = (w - wf) * V[h].f3;
                                             const double2 *A = sA + 3 * k[h];
                                             dv[0] = fma(w - wf, V[h].f1 + V[h].f3, dv[0]);

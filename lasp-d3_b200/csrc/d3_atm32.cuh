@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(ATM_THREADS) k_atm32(KP p, int tile) {
         const double4 xa = p.xs[a];
         const int ta = (int)xa.w;
         const SG &g = p.sg[p.sid[a]];
+        const bool ref = atm_reference_order(p, g, p.sid[a]);
         for (int k = tid; k < ne * NR; k += blockDim.x) yapex[k] = p.Y[(size_t)a * ne * NR + k];
         double dwa[NR];
 #pragma unroll
@@ -236,11 +237,8 @@ __global__ void __launch_bounds__(ATM_THREADS) k_atm32(KP p, int tile) {
                         const float lam_xy = dc6 * is3 * is3;
                         const float u = r0sq[tq * ne + pc.y] * id3;
                         const float g3 = u * u * u * sfu_exp2(sfu_log2(u) * (-1.0f / 3.0f));
-                        // reference scale factors (src/d3_kernel.cu:1282-1290) as pair weights
-                        const bool same = (jq == pc.x);
-                        const bool apex_img = qa | (pc.x == a);
-                        const float w = center ? third : (same ? (qa ? third : 1.0f) : (apex_img ? 0.5f : 1.0f));
-                        const float wf = (force_scaled || center) ? w : (same ? 2.0f : 1.0f);
+                        float w = third, wf = third;
+                        if (!center) atm_weights(jq == pc.x, qa, pc.x == a, ref, force_scaled, w, wf);
                         const float d2 = pa.w;
                         const float irsq = id1 * pb.y * id3;
                         const float ir9 = irsq * ir1 * pb.x * ir3;

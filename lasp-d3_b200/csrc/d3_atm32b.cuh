@@ -292,7 +292,7 @@ struct AtmbXSums2 {
 template <int NR, bool SIMPLE>
 __device__ __forceinline__ void atmb_visit2(const AtmbX2<NR> &X, int k0, float2 d3in, bool act0, bool act1,
                                             const float4 P0, const float4 P1, const float4 *yQ0, const float4 *yQ1,
-                                            const float4 *yrow, int a, float third, bool force_scaled,
+                                            const float4 *yrow, int a, bool ref, bool force_scaled,
                                             AtmbXSums2<SIMPLE> &xt, AtmbYSums2<SIMPLE> &ys) {
     const int k1 = (k0 + 1) & 31;
     const float2 ONE = make_float2(1.0f, 1.0f), M1 = make_float2(-1.0f, -1.0f), M2 = make_float2(-2.0f, -2.0f);
@@ -315,20 +315,18 @@ __device__ __forceinline__ void atmb_visit2(const AtmbX2<NR> &X, int k0, float2 
     const float2 lgu = __fmul2_rn(make_float2(sfu_log2(R0.r0sq * id3.x), sfu_log2(R1.r0sq * id3.y)),
                                   make_float2(8.0f / 3.0f, 8.0f / 3.0f));
     const float2 g3 = make_float2(sfu_exp2(lgu.x), sfu_exp2(lgu.y));
-    // reference scale factors (src/d3_kernel.cu:1282-1290) as pair weights; SIMPLE: no
-    // atom appears twice in the list (cell heights > 2 rc_ATM), every weight is 1
+    // pair weights of repeated atoms; SIMPLE: no atom appears twice in the list (cell heights
+    // > 2 rc_ATM), every weight is 1
     float2 nw, wf;
     if (SIMPLE) {
         wf = make_float2(act0 ? 1.0f : 0.0f, act1 ? 1.0f : 0.0f);
         nw = make_float2(act0 ? -1.0f : 0.0f, act1 ? -1.0f : 0.0f);
     } else {
-        const bool same0 = (X.jx == R0.j), same1 = (X.jx == R1.j);
-        const bool img0 = X.qa | (R0.j == a), img1 = X.qa | (R1.j == a);
-        const float w0 = act0 ? (same0 ? (X.qa ? third : 1.0f) : (img0 ? 0.5f : 1.0f)) : 0.0f;
-        const float w1 = act1 ? (same1 ? (X.qa ? third : 1.0f) : (img1 ? 0.5f : 1.0f)) : 0.0f;
-        nw = make_float2(-w0, -w1);
-        wf = make_float2(act0 ? (force_scaled ? w0 : (same0 ? 2.0f : 1.0f)) : 0.0f,
-                         act1 ? (force_scaled ? w1 : (same1 ? 2.0f : 1.0f)) : 0.0f);
+        float w0, w1, wf0, wf1;
+        atm_weights(X.jx == R0.j, X.qa, R0.j == a, ref, force_scaled, w0, wf0);
+        atm_weights(X.jx == R1.j, X.qa, R1.j == a, ref, force_scaled, w1, wf1);
+        nw = make_float2(act0 ? -w0 : 0.0f, act1 ? -w1 : 0.0f);
+        wf = make_float2(act0 ? wf0 : 0.0f, act1 ? wf1 : 0.0f);
     }
     const float2 d1 = X.d1, d2 = make_float2(P1.z, P1.w);
     const float2 irsq = __fmul2_rn(__fmul2_rn(X.id1, make_float2(Q0.z, Q0.w)), id3);
@@ -427,7 +425,6 @@ __global__ void __launch_bounds__((NBUF == 2 ? ATMB_MAXW : ATMB_MAXW1) * 32, 1) 
     for (int k = tid; k < ne * ne; k += blockDim.x) r0sq[k] = (float)(p.r0ab[k] * p.r0ab[k]);
     static_assert(NR == 5 || NR == 7, "reference counts of the parameter tables");
     const float x16c = (float)(4294967296.0 / 43046721.0); // (4/3)^16
-    const float third = 1.0f / 3.0f;
     const float ratm2f = (float)p.ratm2;
     const bool force_scaled = p.atm_force_scaled != 0;
     const double rc = sqrt(p.ratm2);
@@ -452,6 +449,7 @@ __global__ void __launch_bounds__((NBUF == 2 ? ATMB_MAXW : ATMB_MAXW1) * 32, 1) 
         const SG &g = p.sg[p.sid[a]];
         if ((g.atm_simple != 0) != SIMPLE) continue; // the other instance takes this apex
         constexpr bool simple = SIMPLE;
+        const bool ref = !SIMPLE && atm_reference_order(p, g, p.sid[a]);
         for (int k = tid; k < ne * NR; k += blockDim.x) yapex[k] = p.Y[(size_t)a * ne * NR + k];
         for (int k = tid; k < ATMB_CELLS; k += blockDim.x) cellpos[k] = 0;
         if (tid == 0) s_row = 0;
@@ -748,12 +746,12 @@ __global__ void __launch_bounds__((NBUF == 2 ? ATMB_MAXW : ATMB_MAXW1) * 32, 1) 
                             for (int pq = 0; pq < 2; ++pq)
                                 if (__any_sync(0xffffffffu, a0q[pq] | a1q[pq]))
                                     atmb_visit2<NR, simple>(X, kp[pq], d3p[pq], a0q[pq], a1q[pq], P0q[pq], P1q[pq], yQ0,
-                                                            yQ1, yrow_x, a, third, force_scaled, xt, ys[pq]);
+                                                            yQ1, yrow_x, a, ref, force_scaled, xt, ys[pq]);
                         } else if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
                             for (int pq = 0; pq < 2; ++pq)
                                 atmb_visit2<NR, simple>(X, kp[pq], d3p[pq], a0q[pq], a1q[pq], P0q[pq], P1q[pq], yQ0,
-                                                        yQ1, yrow_x, a, third, force_scaled, xt, ys[pq]);
+                                                        yQ1, yrow_x, a, ref, force_scaled, xt, ys[pq]);
                         }
                         const int src = (lane + 4) & 31;
                         ys[0].shift(src);

@@ -66,6 +66,7 @@ struct SG {
     int stcb_off, stcb_n;     // CN / chain-rule stencil of the same blocks
     int stab_off, stab_n;     // rc_ATM stencil of the same blocks (ATM half lists)
     int atm_simple;           // every cell height > 2 rc_ATM: no atom twice in an ATM list
+    double ratm_frac[3];      // rc_ATM over the cell heights
 };
 
 struct KP {
@@ -97,7 +98,7 @@ struct KP {
     int *bin_cnt, *bin_start, *bin_fill, *order;
     // atoms, binned order
     double4 *xs;
-    int4 *shift;
+    int4 *shift; // lattice shift removed by wrapping; .w height in the cell (atm_before)
     int *bin_s, *orig, *sorted_of;
     double *cn, *w, *dw, *Y;
     double *e2, *g2, *f2, *v2; // two-body: energy, dE/dCN, force[3], virial[6]
@@ -140,6 +141,10 @@ struct KP {
     // atom groups of the two-body pass (d3_pairs.cuh): super-rows, groups and their
     // count, stencil-row slices per group, per-slice partial sums, work counter
     int *anyshift;           // per structure: some atom was given outside the cell
+    unsigned int *span;      // per structure and lattice direction: extent of the positions as
+                             // given (SPAN0 - floor, SPAN0 + ceil of the fractional
+                             // coordinates x 65536, each the largest over the atoms)
+    int atm_ref_order;       // 1: ATM lists in the reference's order (diagnostics)
     const int4 *srows;
     int nsrow;
     int4 *groups;
@@ -152,6 +157,57 @@ __device__ __forceinline__ int floordiv(int a, int b) {
     int q = a / b;
     if ((a % b != 0) && ((a < 0) != (b < 0))) --q;
     return q;
+}
+
+constexpr unsigned int SPAN0 = 1u << 30;
+
+// Order of the ATM half lists. A triplet of lattice points is visited from the apex that
+// comes last in a translation-invariant order: by height along the third lattice vector
+// (T_z, then the wrapped fractional coordinate, kept as an integer in shift.w), equal
+// heights by binned index and (T_y, T_x). Every half list is then the lower half of the ball
+// around its apex: equally long for all apexes, compact, and with 61 % of its entry pairs in
+// range (47 % for the reference's choice of the largest caller index, whose lists are
+// random parts of a ball), and no triplet is visited twice. The reference's image box
+// applies to pairs with the apex only, so where it can cut pairs within rc_ATM its own apex
+// choice decides which triplets exist: then (and for diagnostics) the lists hold j <= a in
+// caller order. 20,000-atom box, ATM pass: FP32 226.5 -> 186.3 ms, FP64 630 -> 581 ms;
+// 96-atom water box, FP32 1.47 -> 1.19 ms.
+__device__ __forceinline__ bool atm_reference_order(const KP &p, const SG &g, int sid) {
+    if (p.atm_ref_order) return true;
+    if (!g.box_mode) return false;
+    bool cut = false;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int extent = (int)(p.span[6 * sid + 2 * k] - SPAN0) + (int)(p.span[6 * sid + 2 * k + 1] - SPAN0);
+        cut |= (int)floor(extent * (1.0 / 65536.0) + g.ratm_frac[k] + 1e-6) > g.half[k];
+    }
+    return cut;
+}
+// key: caller index (ref) or height
+__device__ __forceinline__ int atm_key(const KP &p, bool ref, int j) { return ref ? p.orig[j] : p.shift[j].w; }
+__device__ __forceinline__ bool atm_before(bool ref, int j, int a, int kj, int ka, int Tx, int Ty, int Tz) {
+    if (ref) return kj <= ka;
+    if (Tz != 0) return Tz < 0;
+    if (kj != ka) return kj < ka;
+    if (j != a) return j < a;
+    return Ty != 0 ? Ty < 0 : Tx < 0;
+}
+
+// Weights of a triplet whose entry atoms are equal (same) or are the apex atom (qa, pa): w
+// for energy, dE/dCN and virial, wf for forces. Reference order: its scale factors
+// (src/d3_kernel.cu:1282-1290), applied to forces only when scaled. The engine's order
+// visits each triplet once where the reference visits it 1 to 3 times: w = 1, and wf the
+// sum of the reference's force weights (1, 2, 6 for none, two, three equal atoms).
+template <typename R>
+__device__ __forceinline__ void atm_weights(bool same, bool qa, bool pa, bool ref, bool scaled, R &w, R &wf) {
+    if (ref) {
+        w = same ? (qa ? (R)(1.0 / 3.0) : (R)1) : (qa || pa ? (R)0.5 : (R)1);
+        wf = scaled ? w : (same ? (R)2 : (R)1);
+    } else {
+        const int n = (same ? 1 : 0) + (qa ? 1 : 0) + (pa ? 1 : 0);
+        w = (R)1;
+        wf = scaled || n == 0 ? (R)1 : (n == 1 ? (R)2 : (R)6);
+    }
 }
 
 __device__ __forceinline__ int shard_atom(const KP &p, int w) { return w * p.shard_world + p.shard_rank; }
@@ -258,6 +314,8 @@ __global__ void k_bin(KP p) {
     const SG &g = p.sg[p.sid_in[i]];
     const double x = p.pos_in[3 * i], y = p.pos_in[3 * i + 1], z = p.pos_in[3 * i + 2];
     int s[3], b[3];
+    unsigned int ext[6];
+    int height = 0;
     bool bad = !(isfinite(x) && isfinite(y) && isfinite(z));
     for (int k = 0; k < 3; ++k) {
         double f = x * g.inv[0 * 3 + k] + y * g.inv[1 * 3 + k] + z * g.inv[2 * 3 + k];
@@ -267,18 +325,31 @@ __global__ void k_bin(KP p) {
         }
         double fl = floor(f);
         s[k] = (int)fl;
+        const double q = fmin(fmax(f, -16000.0), 16000.0) * 65536.0;
+        ext[2 * k] = SPAN0 - (int)floor(q);
+        ext[2 * k + 1] = SPAN0 + (int)ceil(q);
         int bk = (int)((f - fl) * g.nb[k]);
         b[k] = min(max(bk, 0), g.nb[k] - 1);
+        height = (int)fmin((f - fl) * 1073741824.0, 1073741823.0); // of the last direction
     }
     if (bad) atomicOr(p.status, ST_BAD_INPUT);
-    if ((s[0] | s[1] | s[2]) != 0) atomicOr(&p.anyshift[p.sid_in[i]], 1);
+    const int st = p.sid_in[i];
+    if ((s[0] | s[1] | s[2]) != 0) atomicOr(&p.anyshift[st], 1);
+    // extents: one atomic per warp where its atoms belong to one structure
+    const unsigned act = __activemask();
+    const bool one = __all_sync(act, st == __shfl_sync(act, st, __ffs(act) - 1));
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        const unsigned int v = one ? __reduce_max_sync(act, ext[k]) : ext[k];
+        if (!one || (threadIdx.x & 31) == __ffs(act) - 1) atomicMax(&p.span[6 * st + k], v);
+    }
     const int bin = g.bin_base + b[0] + g.nb[0] * (b[1] + g.nb[1] * b[2]);
     double xw = x - (s[0] * g.h[0] + s[1] * g.h[3] + s[2] * g.h[6]);
     double yw = y - (s[0] * g.h[1] + s[1] * g.h[4] + s[2] * g.h[7]);
     double zw = z - (s[0] * g.h[2] + s[1] * g.h[5] + s[2] * g.h[8]);
     if (bad) xw = yw = zw = 0.0;
     p.bin_in[i] = bin;
-    p.shift_in[i] = make_int4(s[0], s[1], s[2], 0);
+    p.shift_in[i] = make_int4(s[0], s[1], s[2], height);
     p.xw_in[i] = make_double4(xw, yw, zw, (double)p.type_in[i]);
     atomicAdd(&p.bin_cnt[bin], 1);
 }
@@ -588,7 +659,7 @@ __global__ void k_twobody(KP p) {
 }
 
 // ------------------------------------------------------------------------------------
-// ATM half list: for apex a, entries (j, T) with caller index j <= a, every side in
+// ATM half list: for apex a, entries (j, T) before a (atm_before), every side in
 // [1e-12, rc_ATM^2] (src/d3_kernel.cu:1235-1269). Count pass then fill pass.
 // ------------------------------------------------------------------------------------
 template <bool FILL>
@@ -610,13 +681,15 @@ __global__ void k_atm_list(KP p) {
         return;
     }
     const bool full = p.atm_center != 0;
+    const bool ref = atm_reference_order(p, g, p.sid[a]);
+    const int ka = atm_key(p, ref, a);
     // the image box needs each partner's wrap shift only when some atom was given outside
     // the cell; otherwise the test is on the image alone
     const bool box_pair = g.box_mode && p.anyshift[p.sid[a]];
     traverse(p, g, p.bin_s[a], p.stencils + g.sta_off, g.sta_n, [&](int j, int Tx, int Ty, int Tz, const double3 &sh, bool act) {
         bool keep = false;
         // (act first: j is a valid index only for active lanes)
-        if (act && (full || p.orig[j] <= oa) &&
+        if (act && (full || atm_before(ref, j, a, atm_key(p, ref, j), ka, Tx, Ty, Tz)) &&
             (box_pair ? in_box(g, sa, p.shift[j], Tx, Ty, Tz)
                       : !(g.box_mode && (abs(Tx) > g.half[0] || abs(Ty) > g.half[1] || abs(Tz) > g.half[2])))) {
             const double4 xj = p.xs[j];
@@ -1227,6 +1300,11 @@ struct Engine {
     } atm_occ_cache[12]; // 0, 2, 4 FP64 ATM, 1, 3 mirror, 5 grouped two-body, 8-11 block-pair ATM
     SurrState surr;
     int shard_rank = 0, shard_world = 0; // set by engine_shard_begin
+    int eval_rank = 0, eval_world = 1;   // of the last evaluation
+    Options eval_opt{};                  // its options
+    bool eval_current = false;           // the atoms and geometry on the device are still its own
+    bool extra_known = false;            // extra_visits holds for it
+    unsigned long long extra_visits = 0;
 
     ~Engine() {
         DBuf<double> *ds[] = {&t_cnref, &t_c6, &t_r0, &t_rcov, &t_r2r4, &t_pairA, &pos_in, &cn, &w, &dw, &Y, &e2,
@@ -1467,7 +1545,7 @@ Engine *engine_create(const uint16_t *elements, uint64_t n_elements, uint64_t ma
         e->sg_dev.ensure(max_structs);
         e->out.ensure(10 * max_structs + 3 * N);
         e->status.ensure(1);
-        e->counters.ensure(4);
+        e->counters.ensure(5);
         for (auto &x : e->ev) D3_CUDA(cudaEventCreate(&x));
         e->host_out.resize(10 * max_structs + 3 * N);
         return e;
@@ -1523,6 +1601,7 @@ static std::vector<int> map_types(const Engine *e, const uint16_t *Z, uint64_t n
 // stencils; uploads the records, the stencil rows and the per-atom structure index.
 static void build_structures(Engine *e, int nstruct, const uint64_t *counts, const double *cells,
                              const float *cells_f) {
+    e->eval_current = false;
     std::vector<SG> sg(nstruct);
     std::vector<CellGeom> geoms(nstruct);
     std::vector<int4> rows, srow;
@@ -1546,6 +1625,7 @@ static void build_structures(Engine *e, int nstruct, const uint64_t *counts, con
         // a nonzero lattice vector is at least as long as the smallest height, so with every
         // height above 2 rc_ATM two images of one atom never lie within rc_ATM of an apex
         r.atm_simple = std::min(g.height[0], std::min(g.height[1], g.height[2])) > 2.0 * e->rc_atm * (1.0 + 1e-9);
+        for (int i = 0; i < 3; ++i) r.ratm_frac[i] = e->use_atm ? e->rc_atm / g.height[i] : 0.0;
         int64_t mcb[3];
         r.box_mode = reference_box(cells_f + 9 * k, e->rc_f, e->rc_cn_f, mcb) ? 1 : 0;
         for (int i = 0; i < 3; ++i) r.half[i] = (int)(mcb[i] / 2);
@@ -1617,7 +1697,7 @@ static void build_structures(Engine *e, int nstruct, const uint64_t *counts, con
         D3_CUDA(cudaMemcpy(e->srows.p, srow.data(), sizeof(int4) * srow.size(), cudaMemcpyHostToDevice));
     e->groups.ensure(e->group_bound);
     e->gctl.ensure(6); // [0] groups, [1..5] work counters: CN, two-body, chain, ATM list count, fill
-    e->anyshift.ensure(std::max(1, nstruct));
+    e->anyshift.ensure(7 * (size_t)std::max(1, nstruct)); // flag, then the six extents, per structure
     e->nstruct = nstruct;
     e->nbins_total = bin_base;
     e->sg_dev.ensure(nstruct);
@@ -1642,6 +1722,7 @@ int engine_set_atoms(Engine *e, const double *pos_bohr, const uint16_t *Z, uint6
         D3_CUDA(cudaMemcpyAsync(e->type_in.p, types.data(), sizeof(int) * n, cudaMemcpyHostToDevice, e->stream));
         D3_CUDA(cudaStreamSynchronize(e->stream));
         const bool recount = e->n != n;
+        if (recount) e->eval_current = false;
         e->n = n;
         e->atoms_set = true;
         if (e->cell_set && (recount || e->nstruct != 1)) {
@@ -1693,6 +1774,7 @@ int engine_set_batch(Engine *e, uint64_t nstruct, const uint64_t *counts, const 
         D3_CUDA(cudaMemcpyAsync(e->pos_in.p, pos_bohr, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, e->stream));
         D3_CUDA(cudaMemcpyAsync(e->type_in.p, types.data(), sizeof(int) * n, cudaMemcpyHostToDevice, e->stream));
         D3_CUDA(cudaStreamSynchronize(e->stream));
+        e->eval_current = false;
         e->n = n;
         e->atoms_set = true;
         e->cell_set = true;
@@ -1811,6 +1893,23 @@ static int pairs_occupancy(Engine *e) {
     return c.blocks;
 }
 
+// CTAs that share one apex (systems of few apexes): apexes are equally long, so a pass takes
+// ceil(apexes S / CTAs) waves of items, each an S-th of an apex and the set-up that every
+// split repeats (`setup`, in apexes). The S of the shortest pass; without it 16 and 96 apexes
+// leave most of the 148 SMs idle (FP64 ATM pass 26.8 and 36 ms, with it 0.4 and 3.3 ms).
+static int apex_split(long long apexes, long long ctas, int most, double setup) {
+    int best = 1;
+    double least = 1e300;
+    for (int S = 1; S <= most; ++S) {
+        const double t = (double)((apexes * S + ctas - 1) / ctas) * (1.0 / S + setup);
+        if (t < least * (1.0 - 1e-9)) {
+            least = t;
+            best = S;
+        }
+    }
+    return best;
+}
+
 // CTAs per SM of the FP64 ATM kernel, their shared memory and the splits of an apex
 struct Atm64Shape {
     int ctas, nrows, split;
@@ -1824,11 +1923,7 @@ static Atm64Shape atm64_shape(const Engine *e, int world) {
     const size_t limit = std::min<size_t>(227 * 1024, 228 * 1024 / sh.ctas - 1024) - ATM64_STATIC;
     sh.fixed = atm64_fixed_bytes(e->ne, e->nref, ATM64_THREADS / 32 / sh.ctas, sh.nrows);
     sh.tile_bytes = limit - sh.fixed;
-    const long long apexes = std::max<long long>(1, (long long)e->n / std::max(1, world));
-    const long long items = 6LL * e->dev_sms * sh.ctas;
-    // about six items per CTA, so that systems of few apexes fill the GPU and the last items
-    // are short against the pass (16-atom cell 26.8 -> 0.5 ms, 96 atoms 36 -> 3.4 ms)
-    sh.split = (int)std::max<long long>(1, std::min<long long>(32, (items + apexes - 1) / apexes));
+    sh.split = apex_split(std::max<long long>(1, (long long)e->n / std::max(1, world)), e->dev_sms * sh.ctas, 32, 0.01);
     return sh;
 }
 
@@ -1884,13 +1979,9 @@ static KP make_kp(Engine *e) {
         e->atmb_scratch.ensure((size_t)e->dev_sms * sh.ctas * atmb_scratch_per_cta(sh.mcap));
         p.atmb_mcap = sh.mcap;
         p.YD32 = e->YD32.p;
-        // few apexes (small structures): split each apex's block rows over several CTAs so
-        // that about three work items per CTA exist (every split repeats the apex's entry
-        // sort and set-up: on the 96-atom water box splits 3 / 5 / 7 / 10 / 16 took
-        // 1.60 / 1.48 / 1.78 / 2.13 / 2.77 ms)
         const int ctas = e->dev_sms * sh.ctas;
         p.atmb_split = e->opt.atmb_split > 0 ? std::min(e->opt.atmb_split, 64)
-                                             : std::max(1, std::min(16, (3 * ctas + p.n - 1) / std::max(1, p.n)));
+                                             : apex_split(std::max(1, p.n), ctas, 16, 0.05);
     }
     if (e->use_atm && !p.precision) {
         const Atm64Shape sh = atm64_shape(e, 1);
@@ -1898,6 +1989,7 @@ static KP make_kp(Engine *e) {
     }
     p.atm_force_scaled = e->opt.atm_force_scaled ? 1 : 0;
     p.anyshift = e->anyshift.p;
+    p.span = reinterpret_cast<unsigned int *>(e->anyshift.p + e->nstruct);
     p.srows = e->srows.p;
     p.nsrow = (int)e->srow_host.size();
     p.groups = e->groups.p;
@@ -2038,6 +2130,167 @@ static d3mlp::Net surr_net(const SurrState &S) {
     return net;
 }
 
+// Triplets that the reference's enumeration visits more than once: with two images of an
+// atom of larger caller index than the third it takes either image as the apex, with three
+// images of one atom each. Counts the additional visits of the lists in the engine's order
+// (only asked for with the work counters), one CTA per apex.
+__global__ void k_atm_extra_visits(KP p, unsigned long long *extra) {
+    const int a = blockIdx.x;
+    const int sid = p.sid[a];
+    const SG &g = p.sg[sid];
+    if (g.atm_simple || atm_reference_order(p, g, sid) || p.atm_off[p.n] > p.atm_cap) return;
+    const long long e0 = p.atm_off[a];
+    const int m = (int)(p.atm_off[a + 1] - e0);
+    const double4 xa = p.xs[a];
+    auto pos = [&](int k, int &j) {
+        const int2 ent = p.atm_ent[e0 + k];
+        j = ent.x;
+        const double4 xj = p.xs[j];
+        double sx, sy, sz;
+        image_vec(g, sext8(ent.y & 0xff), sext8((ent.y >> 8) & 0xff), sext8((ent.y >> 16) & 0xff), sx, sy, sz);
+        return make_double3(xj.x + sx - xa.x, xj.y + sy - xa.y, xj.z + sz - xa.z);
+    };
+    unsigned long long more = 0;
+    for (int x = threadIdx.x; x < m; x += blockDim.x) {
+        int jx;
+        const double3 v = pos(x, jx);
+        for (int y = 0; y < x; ++y) {
+            const int jy = p.atm_ent[e0 + y].x;
+            if (jx != jy && jx != a && jy != a) continue;
+            int j;
+            const double3 u = pos(y, j);
+            const double rx = v.x - u.x, ry = v.y - u.y, rz = v.z - u.z;
+            const double d3 = fma(rx, rx, fma(ry, ry, rz * rz));
+            if (d3 > p.ratm2 || d3 < 1e-12) continue;
+            if (jx == jy && jx == a)
+                more += 2;
+            else { // the repeated atom and the other one
+                const int r = jx == jy ? jx : a, o = jx == jy ? a : (jx == a ? jy : jx);
+                more += p.orig[r] > p.orig[o] ? 1 : 0;
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) more += __shfl_xor_sync(0xffffffffu, more, o);
+    if ((threadIdx.x & 31) == 0 && more) atomicAdd(extra, more);
+}
+
+// additional visits of the last evaluation's triplets in the reference's enumeration
+static unsigned long long engine_extra_visits(Engine *e) {
+    if (e->extra_known) return e->extra_visits;
+    bool weighted = false;
+    for (const SG &q : e->sg) weighted |= !q.atm_simple;
+    unsigned long long n = 0;
+    if (e->use_atm && weighted && e->eval_current && !(e->opt.atm_surrogate && e->surr.loaded)) {
+        KP p = make_kp(e);
+        unsigned long long *d = e->counters.p + 4;
+        D3_CUDA(cudaMemset(d, 0, sizeof(*d)));
+        k_atm_extra_visits<<<p.n, 128>>>(p, d);
+        D3_CUDA(cudaGetLastError());
+        D3_CUDA(cudaMemcpy(&n, d, sizeof(*d), cudaMemcpyDeviceToHost));
+    }
+    return n;
+}
+
+// ATM half lists of every apex (of the flagged ones in centre mode)
+static void launch_atm_lists(Engine *e, const KP &p, cudaStream_t s) {
+    const int n = p.n, T = 256;
+    const int gb = (n + T - 1) / T;
+    const int gw = (int)(((long long)n * 32 + T - 1) / T);
+    if (p.gslices > 0) {
+        const size_t sm = PAIRS_WARPS * 32 * (sizeof(double4) + sizeof(int));
+        k_atm_list_g<false><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(p, e->gctl.p + 4);
+        k_atm_list_prefix<<<gb, T, 0, s>>>(p);
+        k_scan<long long, int><<<1, 1024, 0, s>>>(p.atm_cnt, p.atm_off, n);
+        k_atm_list_g<true><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(p, e->gctl.p + 5);
+    } else {
+        k_atm_list<false><<<gw, T, 0, s>>>(p);
+        k_scan<long long, int><<<1, 1024, 0, s>>>(p.atm_cnt, p.atm_off, n);
+        k_atm_list<true><<<gw, T, 0, s>>>(p);
+    }
+}
+
+// ATM triplets over the half lists; surr: centre mode of the surrogate fallback
+template <int NR>
+static void launch_atm_triplets(Engine *e, const KP &p0, cudaStream_t s, bool surr) {
+    KP p = p0;
+    const int n = p.n;
+    D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
+    if (p.precision) {
+        const size_t fixed = (size_t)p.ne * NR * sizeof(double) + ((p.ne * p.ne + 3) & ~3) * sizeof(float) +
+                             ATM_PERM_CAP * sizeof(unsigned short) + 11 * ATM_THREADS * sizeof(double);
+        const size_t per = 2 * sizeof(float4) + sizeof(int2) + (size_t)p.ne * 2 * sizeof(float4);
+        const int tmax = (int)std::max<size_t>(32, std::min<size_t>(256, (100 * 1024 - fixed) / per)) & ~31;
+        const int tile = e->opt.atm_tile > 0 ? std::min(tmax, std::max(32, e->opt.atm_tile & ~31)) : std::min(tmax, 128);
+        const size_t sm = (size_t)tile * per + fixed;
+        const AtmbShape shb = blockpair_shape(e);
+        const int nwb = shb.warps;
+        if (nwb > 0 && !surr) {
+            // lists up to shb.mcap entries: block-pair schedule; longer ones below
+            const size_t smb =
+                atmb_smem_fixed(p.ne, NR, shb.mcap) + (size_t)nwb * atmb_smem_warp(p.ne, NR, shb.nbuf);
+            // one launch per apex kind present: weight-free structures (every cell
+            // height above 2 rc_ATM) and the others
+            bool kind[2] = {false, false};
+            for (const SG &q : e->sg) kind[q.atm_simple ? 1 : 0] = true;
+            const int grid = e->dev_sms * shb.ctas;
+            for (int k = 1; k >= 0; --k) {
+                if (!kind[k]) continue;
+                if (k == 0 && kind[1]) D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
+                launch_blockpair<NR>(e, p, s, shb, k == 1, grid, smb);
+            }
+            D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
+            p.atm_min_m = shb.mcap;
+        }
+        const void *fn = surr ? (const void *)k_atm32<NR, true> : (const void *)k_atm32<NR, false>;
+        const int blocks_per_sm = atm_occupancy(e, surr ? 3 : 1, sm, fn);
+        const int per_sm = e->opt.atm_ctas_per_sm > 0 ? std::min(e->opt.atm_ctas_per_sm, blocks_per_sm) : blocks_per_sm;
+        const int grid = std::max(1, std::min(n, e->dev_sms * std::max(1, per_sm)));
+        if (surr)
+            k_atm32<NR, true><<<grid, ATM_THREADS, sm, s>>>(p, tile);
+        else
+            k_atm32<NR, false><<<grid, ATM_THREADS, sm, s>>>(p, tile);
+    } else {
+        launch_atm64<NR>(e, p, s, surr);
+    }
+}
+
+// Diagnostics in the reference's apex convention: the lists and the ATM terms of the last
+// evaluation again, with the entries j <= a in caller order (the energies, forces and dE/dCN
+// summed over an atom's apex and entry shares are the same up to rounding).
+static void atm_reference_pass(Engine *e) {
+    if (!e->use_atm || !e->eval_current || (e->eval_opt.atm_surrogate && e->surr.loaded)) return;
+    D3_CUDA(cudaDeviceSynchronize());
+    e->extra_visits = engine_extra_visits(e);
+    e->extra_known = true; // the lists are about to change their order
+    const Options now = e->opt;
+    e->opt = e->eval_opt;
+    const cudaStream_t s = e->stream;
+    const size_t n = e->n;
+    for (int attempt = 0; attempt < 4; ++attempt) {
+        KP p = make_kp(e);
+        p.shard_rank = e->eval_rank;
+        p.shard_world = e->eval_world;
+        p.atm_ref_order = 1;
+        p.counters = nullptr;
+        double *sums[] = {p.ea, p.ga, p.fa, p.va, p.eb, p.gb, p.fb};
+        const int width[] = {1, 1, 3, 6, 1, 1, 3};
+        for (int k = 0; k < 7; ++k) D3_CUDA(cudaMemsetAsync(sums[k], 0, sizeof(double) * width[k] * n, s));
+        D3_CUDA(cudaMemsetAsync(e->gctl.p + 4, 0, 2 * sizeof(int), s));
+        launch_atm_lists(e, p, s);
+        if (e->nref == 5)
+            launch_atm_triplets<5>(e, p, s, false);
+        else
+            launch_atm_triplets<7>(e, p, s, false);
+        long long need = 0;
+        D3_CUDA(cudaMemcpyAsync(&need, e->atm_off.p + n, sizeof(long long), cudaMemcpyDeviceToHost, s));
+        D3_CUDA(cudaStreamSynchronize(s));
+        if (need <= e->atm_cap) break;
+        e->atm_cap = (long long)(need * 1.1) + 1024;
+        e->atm_ent.ensure((size_t)e->atm_cap);
+    }
+    e->opt = now;
+}
+
 // stage 0: the whole evaluation; stage 1: everything up to the summed dE/dCN (written to
 // G_ext when given); stage 2: chain rule (dE/dCN read from G_ext), forces and reductions.
 // Stages 1 and 2 with an all-reduce of dE/dCN between them make a sharded evaluation.
@@ -2051,9 +2304,14 @@ static void launch_all(Engine *e, const KP &p0, cudaStream_t s, int stage = 0, d
     cudaEvent_t *ev = e->ev;
     double *Gsum = G_ext ? G_ext : e->G.p;
     if (stage != 2) {
+        e->eval_rank = p.shard_rank;
+        e->eval_world = p.shard_world;
+        e->eval_opt = e->opt;
+        e->eval_current = true;
+        e->extra_known = false;
         D3_CUDA(cudaEventRecord(ev[0], s));
         D3_CUDA(cudaMemsetAsync(p.counters, 0, sizeof(unsigned long long) * 4, s));
-        D3_CUDA(cudaMemsetAsync(p.anyshift, 0, sizeof(int) * p.nstruct, s));
+        D3_CUDA(cudaMemsetAsync(p.anyshift, 0, 7 * sizeof(int) * p.nstruct, s));
         D3_CUDA(cudaMemsetAsync(p.bin_cnt, 0, sizeof(int) * p.nbins_total, s));
         D3_CUDA(cudaMemsetAsync(p.bin_fill, 0, sizeof(int) * p.nbins_total, s));
         k_bin<<<gb, T, 0, s>>>(p);
@@ -2134,57 +2392,10 @@ static void launch_all(Engine *e, const KP &p0, cudaStream_t s, int stage = 0, d
             pc.atm_napex = S.napex.p;
             pc.surr_flag = S.flag.p;
         }
-        if (e->use_atm && p.gslices > 0) {
-            const size_t sm = PAIRS_WARPS * 32 * (sizeof(double4) + sizeof(int));
-            k_atm_list_g<false><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(pc, e->gctl.p + 4);
-            k_atm_list_prefix<<<gb, T, 0, s>>>(pc);
-            k_scan<long long, int><<<1, 1024, 0, s>>>(p.atm_cnt, p.atm_off, n);
-            k_atm_list_g<true><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(pc, e->gctl.p + 5);
-        } else if (e->use_atm) {
-            k_atm_list<false><<<gw, T, 0, s>>>(pc);
-            k_scan<long long, int><<<1, 1024, 0, s>>>(p.atm_cnt, p.atm_off, n);
-            k_atm_list<true><<<gw, T, 0, s>>>(pc);
-        }
+        if (e->use_atm) launch_atm_lists(e, pc, s);
         D3_CUDA(cudaEventRecord(ev[4], s));
         if (e->use_atm) {
-            D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
-            if (p.precision) {
-                const size_t fixed = (size_t)p.ne * NR * sizeof(double) + ((p.ne * p.ne + 3) & ~3) * sizeof(float) +
-                                     ATM_PERM_CAP * sizeof(unsigned short) + 11 * ATM_THREADS * sizeof(double);
-                const size_t per = 2 * sizeof(float4) + sizeof(int2) + (size_t)p.ne * 2 * sizeof(float4);
-                const int tmax = (int)std::max<size_t>(32, std::min<size_t>(256, (100 * 1024 - fixed) / per)) & ~31;
-                const int tile = e->opt.atm_tile > 0 ? std::min(tmax, std::max(32, e->opt.atm_tile & ~31)) : std::min(tmax, 128);
-                const size_t sm = (size_t)tile * per + fixed;
-                const AtmbShape shb = blockpair_shape(e);
-                const int nwb = shb.warps;
-                if (nwb > 0 && !surr) {
-                    // lists up to shb.mcap entries: block-pair schedule; longer ones below
-                    const size_t smb =
-                        atmb_smem_fixed(p.ne, NR, shb.mcap) + (size_t)nwb * atmb_smem_warp(p.ne, NR, shb.nbuf);
-                    // one launch per apex kind present: weight-free structures (every cell
-                    // height above 2 rc_ATM) and the others
-                    bool kind[2] = {false, false};
-                    for (const SG &q : e->sg) kind[q.atm_simple ? 1 : 0] = true;
-                    const int grid = e->dev_sms * shb.ctas;
-                    for (int k = 1; k >= 0; --k) {
-                        if (!kind[k]) continue;
-                        if (k == 0 && kind[1]) D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
-                        launch_blockpair<NR>(e, p, s, shb, k == 1, grid, smb);
-                    }
-                    D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
-                    pc.atm_min_m = shb.mcap;
-                }
-                const void *fn = surr ? (const void *)k_atm32<NR, true> : (const void *)k_atm32<NR, false>;
-                const int blocks_per_sm = atm_occupancy(e, surr ? 3 : 1, sm, fn);
-                const int per_sm = e->opt.atm_ctas_per_sm > 0 ? std::min(e->opt.atm_ctas_per_sm, blocks_per_sm) : blocks_per_sm;
-                const int grid = std::max(1, std::min(n, e->dev_sms * std::max(1, per_sm)));
-                if (surr)
-                    k_atm32<NR, true><<<grid, ATM_THREADS, sm, s>>>(pc, tile);
-                else
-                    k_atm32<NR, false><<<grid, ATM_THREADS, sm, s>>>(pc, tile);
-            } else {
-                launch_atm64<NR>(e, pc, s, surr);
-            }
+            launch_atm_triplets<NR>(e, pc, s, surr);
             if (surr) k_desc_bwd<NR><<<gw, T, 0, s>>>(p, sd);
         }
         D3_CUDA(cudaEventRecord(ev[5], s));
@@ -2222,7 +2433,10 @@ int engine_pass_times(Engine *e, float *ms, int cap, unsigned long long *counter
     D3_CUDA(cudaEventSynchronize(e->ev[Engine::NEV - 1]));
     int k = 0;
     for (; k < Engine::NEV - 1 && k < cap; ++k) D3_CUDA(cudaEventElapsedTime(&ms[k], e->ev[k], e->ev[k + 1]));
-    if (counters) D3_CUDA(cudaMemcpy(counters, e->counters.p, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost));
+    if (counters) {
+        D3_CUDA(cudaMemcpy(counters, e->counters.p, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost));
+        counters[0] += 2 * engine_extra_visits(e);
+    }
     return k;
 }
 
@@ -2407,6 +2621,7 @@ int engine_debug_pass_terms(Engine *e, double *out) {
     // virial[6]; chain-rule force[3], virial[6]; virials as xx yy zz xy xz yz, already
     // scaled by the pass's volume factor
     const uint64_t n = e->n;
+    atm_reference_pass(e);
     std::vector<int> orig(n);
     D3_CUDA(cudaStreamSynchronize(e->stream));
     D3_CUDA(cudaMemcpy(orig.data(), e->orig.p, sizeof(int) * n, cudaMemcpyDeviceToHost));
@@ -2434,6 +2649,7 @@ int64_t engine_debug_atm_pairs(Engine *e, int64_t *outp, int64_t cap) {
     // returns (apex, j, Tref_x, Tref_y, Tref_z) rows in caller indices and reference shifts
     if (!e->use_atm) return 0;
     const uint64_t n = e->n;
+    atm_reference_pass(e);
     std::vector<long long> off(n + 1);
     std::vector<int> orig(n);
     std::vector<int4> sh(n);

@@ -556,8 +556,8 @@ __global__ void k_group_reduce(KP p, int what) {
     }
 }
 
-// ATM half lists on atom groups (rc_ATM stencil): for apex a the entries (j, T) with j <= a in
-// caller order (all of them in centre mode) and 1e-12 <= r^2 <= rc_ATM^2, the distance
+// ATM half lists on atom groups (rc_ATM stencil): for apex a the entries (j, T) before a
+// (atm_before; all of them in centre mode) and 1e-12 <= r^2 <= rc_ATM^2, the distance
 // evaluated as the per-apex kernel does (x_a - (x_j + T h)). Count pass: counts per
 // (stencil slice, apex) into the partial array; k_atm_list_prefix turns them into offsets
 // within the apex and the apex totals; fill pass: every lane writes its apex's entries of
@@ -588,15 +588,18 @@ __global__ void __launch_bounds__(PAIRS_WARPS * 32, 2) k_atm_list_g(KP p, int *w
                 take = false;
         }
         const bool box_pair = g.box_mode && p.anyshift[it.sr.x];
+        const bool ref = atm_reference_order(p, g, it.sr.x);
+        const int ka = take ? atm_key(p, ref, a) : 0;
         long long pos = 0;
         int count = 0;
         if (FILL && take) pos = p.atm_off[a] + gcnt[(size_t)it.sl * p.n + a];
         group_ranges<double, double4>(p, it, p.stencils + g.stab_off, g.stab_n, box_pair, xa,
                                       [&](int base, int m, double, double, double, int px, int Ty, int Tz) {
+            if (!full && !ref && Tz > 0) return; // images that come after every apex
             __syncwarp();
             if (lane < m) {
                 sP[lane] = p.xs[base + lane];
-                sO[lane] = p.orig[base + lane];
+                sO[lane] = atm_key(p, ref, base + lane);
             }
             __syncwarp();
             if (!take) return;
@@ -604,7 +607,7 @@ __global__ void __launch_bounds__(PAIRS_WARPS * 32, 2) k_atm_list_g(KP p, int *w
             const double shy = px * g.h[1] + Ty * g.h[4] + Tz * g.h[7];
             const double shz = px * g.h[2] + Ty * g.h[5] + Tz * g.h[8];
             for (int jj = 0; jj < m; ++jj) {
-                if (!full && sO[jj] > oa) continue;
+                if (!full && !atm_before(ref, base + jj, a, sO[jj], ka, px, Ty, Tz)) continue;
                 if (box_pair && !in_box(g, sa, p.shift[base + jj], px, Ty, Tz)) continue;
                 const double4 xj = sP[jj];
                 const double dx = xa.x - (xj.x + shx), dy = xa.y - (xj.y + shy), dz = xa.z - (xj.z + shz);
