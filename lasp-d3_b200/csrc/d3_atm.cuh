@@ -7,13 +7,18 @@
 // order (entries j <= a in caller order) this is its (b, T_b, c, T_c) loop with c <= b
 // (src/d3_kernel.cu:1235-1327). Repeated atoms change the weights (atm_weights).
 //
-// Schedule: persistent CTAs pull (apex, split) items from a work counter; the splits of an apex share its entries x (rows) between CTAs, so that systems of
-// few apexes fill the GPU. A warp owns one row x at a time. It tests x against the staged
-// partners 32 at a time (FP32 positions; pairs near a limit again in FP64) and queues the
-// ones in range; when 32 are queued, all 32 lanes visit one partner y each. Every visit
-// slot then does work whatever the shape of the lists, and everything that belongs to x is
-// the same in all lanes, so its sums cost one warp reduction per row and partner tile.
-// Every unordered pair is visited from both of its entries, so nothing is added to y.
+// Schedule: persistent CTAs pull (apex, split) items from a work counter; the splits of an
+// apex share its entries x (rows) between CTAs, so that systems of few apexes fill the GPU.
+// The entries are sorted along a Hilbert curve and staged in shared memory as partners, 32
+// consecutive ones a chunk with a bounding sphere. A warp owns one row x at a time:
+//  1. each lane compares x with the sphere of one chunk: out of range, all in range, or mixed;
+//  2. chunks all in range are visited as they are, one partner y per lane;
+//  3. partners of mixed chunks are tested (FP32 positions; pairs near a limit again in FP64),
+//     the ones in range are queued, and whole warps of them are visited.
+// Nearly every visit slot then does work whatever the shape of the lists, and everything
+// that belongs to x is the same in all lanes, so its sums cost one warp reduction per row
+// and partner tile. Every unordered pair is visited from both of its entries, so nothing is
+// added to y.
 //
 // The queue has eight classes, k mod 8 for partner k, and a class feeds the four lanes l
 // with l mod 8 equal to it: the eight lanes that share a 128-byte wavefront of a 16-byte
@@ -30,11 +35,15 @@
 // damping, since 6 x fd = 1 - fd). That is the reference's angular and damping derivative
 // (:1367-1392) regrouped: 83 FP64 operations a visit, two visits a triplet.
 //
-// Bound: the FP64 pipe (a warp instruction takes two cycles of a scheduler's pipe), 40 %
-// busy on the 20,000-atom box; the rest is latency of the test and queue steps.
-// ATM pass on a B200, one thread per entry with a private partner mask before -> now:
-// 16-atom metal cell 26.8 -> 0.51 ms, 96-atom water box 36.2 -> 3.4 ms (their few apexes
-// are split over all CTAs), 777 atoms 49.4 -> 25.5 ms, 20,000-atom box 745 -> 630 ms.
+// Bound: instruction issue, where an FP64 instruction counts twice (its pipe takes a warp in
+// two cycles). A visit alone costs 200 cycles of a scheduler (83 FP64 and 24 other
+// instructions), on the 20,000-atom box 310 with everything else: of the ATM pass 31 % are
+// visits of whole chunks, 37 % of queued partners (15 % of their lanes idle), 13 % range
+// tests, 10 % row set-up and sums, 4 % set-up of the apex.
+// ATM pass on a B200, one thread per entry with a private partner mask -> this kernel:
+// 16-atom metal cell 26.8 -> 0.38 ms, 96-atom water box 36.2 -> 2.65 ms (their few apexes
+// are split over all CTAs), 777 atoms 49.4 -> 20.7 ms, 2,000 atoms 73.3 -> 50.0 ms,
+// 20,000-atom box 745 -> 441 ms.
 
 // ---- refined reciprocal roots ------------------------------------------------------
 __device__ __forceinline__ double rsqrt_nr(double x) {
@@ -77,11 +86,15 @@ __device__ __forceinline__ double rcbrt_nr2(double x) {
     return fma(z * fma(-x * z, z * z, 1.0), 1.0 / 3.0, z);
 }
 
-constexpr int ATM64_THREADS = 384;  // threads of all CTAs of an SM together
-constexpr int ATM64_ROWS = 4096;    // entries whose rows are listed at once, over the CTAs of an SM
-constexpr int ATM64_SEG = 128;      // partners tested before the queue is looked at
-constexpr int ATM64_QCAP = 64;      // queue slots per class and warp (at least 8 + ATM64_SEG / 8)
-constexpr int ATM64_STATIC = 2048;  // bytes left for the static arrays
+constexpr int ATM64_THREADS = 512;  // threads of all CTAs of an SM together
+constexpr int ATM64_ROWS = 4096;    // entries set up at once (longer lists: in parts)
+constexpr int ATM64_CHUNKS = 64;    // chunks of 32 partners in a tile at most
+constexpr int ATM64_SEG = 4;        // chunks tested together
+constexpr int ATM64_GROUP = 32;     // mixed chunks of a row queued at once (a multiple of ATM64_SEG)
+constexpr int ATM64_QCAP = 4 * ATM64_GROUP; // queue slots per class and warp
+constexpr int ATM64_LIST = ATM64_CHUNKS + ATM64_SEG; // a row's chunks: all in range from the front, mixed from the back
+constexpr int ATM64_CELLS = 4096;   // sort cells: 16^3, fewer for short lists
+constexpr int ATM64_STATIC = 5120;  // bytes left for the static arrays
 
 // apex kinds, one instance each: weight-free structures (no atom twice in a list), the
 // others, and the surrogate fallback's centre mode (apexes from p.atm_apex, full lists,
@@ -95,19 +108,40 @@ __host__ __device__ constexpr int atm64_rowq(int NR) { return NR == 5 ? 3 : 5; }
 __host__ __device__ constexpr size_t atm64_partner_bytes(int NR, int types) {
     return 3 * sizeof(double2) + sizeof(float4) + (size_t)types * atm64_rowq(NR) * sizeof(double2);
 }
-__host__ __device__ inline size_t atm64_fixed_bytes(int ne, int NR, int warps, int nrows) {
+// tile bytes: the partners, 32 far positions (the first of them the dummy partner of idle
+// lanes, with a record and rows of its own), the chunk bounds
+__host__ __device__ constexpr size_t atm64_tile_fixed(int NR, int types) {
+    return atm64_partner_bytes(NR, types) + 31 * sizeof(float4) + 2 * ATM64_CHUNKS * sizeof(float4);
+}
+__host__ __device__ inline size_t atm64_fixed_bytes(int ne, int NR, int warps) {
     size_t b = (size_t)((ne * NR + 1) & ~1) * sizeof(double) + (size_t)((ne * ne + 1) & ~1) * sizeof(double);
-    b += (size_t)warps * 8 * ATM64_QCAP * sizeof(unsigned short);
-    b += (size_t)nrows * sizeof(unsigned short) + (size_t)((2 * ne + 2 + 3) & ~3) * sizeof(int);
+    b += (size_t)warps * (8 * ATM64_QCAP + ATM64_LIST * sizeof(unsigned short));
+    b += (size_t)((2 * ne + 2 + 3) & ~3) * sizeof(int);
     return (b + 15) & ~(size_t)15;
 }
 
-// one entry of the apex as a row
-struct Atm64Row {
+// one entry of the apex: the first three words are its record as a partner
+struct __align__(16) Atm64Row {
     double v[3], id, p, g; // position from the apex, 1/d, sqrt(C6)/r^3, (r0^2/d)^(8/3)
     double lam_ea, lam_ae; // dC6/dCN over C6: of the entry, of the apex
-    int j, t;
+    int j, t, k, pad;      // atom, type, entry number
+    float f[4];            // rounded position
 };
+// scratch of one CTA: the entries, and the rows of its split by type with their C6 weights
+struct Atm64Scratch {
+    Atm64Row entries[ATM64_ROWS];
+    struct Row {
+        Atm64Row e;
+        double w[MAX_NREF + 1], dw[MAX_NREF + 1];
+    } rows[ATM64_ROWS];
+};
+
+// position of an entry relative to the apex
+__device__ __forceinline__ double3 atm64_pos(const KP &p, const SG &g, const double4 &xa, const int2 ent, const double4 &xj) {
+    double sx, sy, sz;
+    image_vec(g, sext8(ent.y & 0xff), sext8((ent.y >> 8) & 0xff), sext8((ent.y >> 16) & 0xff), sx, sy, sz);
+    return make_double3(xj.x + sx - xa.x, xj.y + sy - xa.y, xj.z + sz - xa.z);
+}
 
 // per-entry set-up (FP64 C6 of the apex pair, its CN derivatives, damping ratio)
 template <int NR>
@@ -117,11 +151,10 @@ __device__ __forceinline__ Atm64Row atm64_entry(const KP &p, const SG &g, const 
     const double4 xj = p.xs[ent.x];
     r.j = ent.x;
     r.t = (int)xj.w;
-    double sx, sy, sz;
-    image_vec(g, sext8(ent.y & 0xff), sext8((ent.y >> 8) & 0xff), sext8((ent.y >> 16) & 0xff), sx, sy, sz);
-    r.v[0] = xj.x + sx - xa.x;
-    r.v[1] = xj.y + sy - xa.y;
-    r.v[2] = xj.z + sz - xa.z;
+    const double3 v = atm64_pos(p, g, xa, ent, xj);
+    r.v[0] = v.x;
+    r.v[1] = v.y;
+    r.v[2] = v.z;
     const double d = r.v[0] * r.v[0] + r.v[1] * r.v[1] + r.v[2] * r.v[2];
     const double ir = rsqrt_nr2(d);
     r.id = ir * ir;
@@ -134,6 +167,9 @@ __device__ __forceinline__ Atm64Row atm64_entry(const KP &p, const SG &g, const 
     r.p = c6 * is * ir * r.id;
     const double u = r0a[r.t] * r.id;
     r.g = u * u * u * rcbrt_nr2(u);
+    r.f[0] = (float)v.x;
+    r.f[1] = (float)v.y;
+    r.f[2] = (float)v.z;
     r.lam_ea = r.lam_ae = 0;
     if (derivatives) {
         const double *yq = p.Y + ((size_t)r.j * p.ne + (int)xa.w) * NR; // dC6_ae/dCN_a = y_{e,ta} . dw_a
@@ -150,6 +186,11 @@ __device__ __forceinline__ Atm64Row atm64_entry(const KP &p, const SG &g, const 
     return r;
 }
 
+// a value that all lanes agree on, through the warp reduction whose result the hardware
+// keeps once per warp: loops bounded by it need no divergence checks at every vote and
+// shuffle inside
+__device__ __forceinline__ int warp_uniform(int v) { return (int)__reduce_max_sync(0xffffffffu, v); }
+
 // one exchange of the row reduction: keep v on the lower lanes and w on the upper ones of
 // each pair `o` apart, adding what the other lane holds of it
 __device__ __forceinline__ double atm64_fold(double v, double w, int o) {
@@ -157,7 +198,7 @@ __device__ __forceinline__ double atm64_fold(double v, double w, int o) {
     return (up ? w : v) + __shfl_xor_sync(0xffffffffu, up ? v : w, o);
 }
 // sums of eight values over the warp; lane l returns the sum of value ((l >> 2) & 7) with
-// its three bits reversed, i.e. value i is on lane atm64_lane(i)
+// its three bits reversed
 __device__ __forceinline__ double atm64_reduce8(const double v[8]) {
     double a[4], b[2];
 #pragma unroll
@@ -168,12 +209,53 @@ __device__ __forceinline__ double atm64_reduce8(const double v[8]) {
     c += __shfl_xor_sync(0xffffffffu, c, 2);
     return c + __shfl_xor_sync(0xffffffffu, c, 1);
 }
-__device__ __forceinline__ constexpr int atm64_lane(int i) {
-    return ((i & 4) << 2) | ((i & 2) << 2) | ((i & 1) << 2);
+
+// Row sums in shared memory: [0..6] the reduced sums, then v_x, 1, 0, lam_ae, lam_ea and the
+// weighted kind's virial sums. Output of lane l from entries S, A, B, U, V, M (s_rule) and
+// coefficients c (s_coef): c0 M sum0 + c1 sum1 + c2 S A B - c3 (U B + V A).
+//   0 energy share of the apex (E/3 per pair, half of it per visit), 1 its dE/dCN, 2..4 its
+//   force -f1 v_x, 5..10 virial f r (x) r with the x-y side's cross part split evenly between
+//   the two visits of a pair (xx yy zz xy xz yz), 11..15 energy, dE/dCN and force of the entry
+enum { ATM64_SV = 8, ATM64_S1 = 11, ATM64_S0 = 12, ATM64_SAE = 13, ATM64_SEA = 14, ATM64_SVIR = 15, ATM64_SR = 20 };
+__device__ inline void atm64_rules(bool weighted, int l, unsigned long long &rule, double c[4]) {
+    const int Z = ATM64_S0;
+    int q[6] = {Z, Z, Z, Z, Z, Z}; // S A B U V M
+    c[0] = c[1] = c[2] = c[3] = 0;
+    if (l == 0 || l == 11) {
+        c[0] = l == 0 ? -1.0 / 6.0 : -1.0 / 3.0;
+        q[5] = ATM64_S1;
+    } else if (l == 1 || l == 12) {
+        c[0] = -0.5;
+        q[5] = l == 1 ? ATM64_SAE : ATM64_SEA;
+        if (l == 12) c[1] = -0.5;
+    } else if (l < 5) {
+        c[2] = -1.0;
+        q[0] = 6;
+        q[1] = ATM64_SV + l - 2;
+        q[2] = ATM64_S1;
+    } else if (l < 11) {
+        const int a = l < 8 ? l - 5 : (l < 10 ? 0 : 1), b = l < 8 ? a : (l == 8 ? 1 : 2);
+        const int vir = weighted ? (int)ATM64_SVIR : 2;
+        c[2] = 1.0;
+        c[3] = 0.5;
+        q[0] = vir;
+        q[1] = ATM64_SV + a;
+        q[2] = ATM64_SV + b;
+        q[3] = vir + 1 + a;
+        q[4] = vir + 1 + b;
+    } else {
+        c[2] = c[3] = 1.0;
+        q[0] = 2;
+        q[1] = ATM64_SV + l - 13;
+        q[2] = ATM64_S1;
+        q[3] = 3 + l - 13;
+    }
+    rule = 0;
+    for (int k = 0; k < 6; ++k) rule |= (unsigned long long)q[k] << (8 * k);
 }
 
 // One visit: triplet (apex, x, y) with x in the arguments and y in the staged records A and
-// R. Branch-free, so that two of them overlap.
+// R. Branch-free.
 struct Atm64Visit {
     double E, lam, f1, f3, vx, vy, vz; // -E, dC6_xy/dCN_x over C6_xy, force scalars, y
 };
@@ -222,28 +304,40 @@ __device__ __forceinline__ void atm64_visit(double vx, double vy, double vz, dou
 }
 
 template <int NR, int KIND>
-__global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Row *scratch, int nrows, int tile_bytes, int tile_max) {
+__global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch *scratch, int tile_bytes, int tile_max) {
     extern __shared__ __align__(16) unsigned char sm64[];
     constexpr int RQ = atm64_rowq(NR);
     const int ne = p.ne, nw = blockDim.x >> 5;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double *yapex = reinterpret_cast<double *>(sm64);              // [ne][NR]
-    double *r0sq = yapex + ((ne * NR + 1) & ~1);                   // [ne][ne] r0ab^2
+    double *yapex = reinterpret_cast<double *>(sm64);                 // [ne][NR]
+    double *r0sq = yapex + ((ne * NR + 1) & ~1);                      // [ne][ne] r0ab^2
     int *toff = reinterpret_cast<int *>(r0sq + ((ne * ne + 1) & ~1)); // [ne + 1] rows of each type, [ne] fill positions
     int *tpos = toff + ne + 1;
-    unsigned short *rowperm = reinterpret_cast<unsigned short *>(toff + ((2 * ne + 2 + 3) & ~3)); // [nrows]
-    unsigned short *queue = rowperm + nrows + warp * 8 * ATM64_QCAP; // [slot][class]
-    unsigned char *area = sm64 + atm64_fixed_bytes(ne, NR, nw, nrows);
-    __shared__ int s_item, s_row;
-    __shared__ double red[ATM64_THREADS / 32][11];
-    if (p.atm_off[p.n] > p.atm_cap) return; // list overflowed: the host grows it and re-runs
+    unsigned char *queue = reinterpret_cast<unsigned char *>(toff + ((2 * ne + 2 + 3) & ~3)) +
+                           (size_t)warp * (8 * ATM64_QCAP + ATM64_LIST * sizeof(unsigned short)); // [slot][class]
+    unsigned short *list = reinterpret_cast<unsigned short *>(queue + 8 * ATM64_QCAP);             // [ATM64_LIST]
+    unsigned char *area = sm64 + atm64_fixed_bytes(ne, NR, nw);
+    int *cells = reinterpret_cast<int *>(area); // [ATM64_CELLS] while the entries are sorted
+    __shared__ int s_item, s_row, s_tot[ATM64_THREADS / 32];
+    __shared__ double red[ATM64_THREADS / 32][11], s_sums[ATM64_THREADS / 32][ATM64_SR], s_coef[16][4];
+    __shared__ unsigned long long s_rule[16];
+    double *sr = s_sums[warp];
+    if (tid < 16) atm64_rules(KIND == ATM64_WEIGHTED, tid, s_rule[tid], s_coef[tid]);
+    if (lane == 0) {
+        sr[ATM64_S1] = 1.0;
+        sr[ATM64_S0] = 0.0;
+    }
+    if (warp_uniform(p.atm_off[p.n] > p.atm_cap ? 1 : 0)) return; // list overflowed: the host grows it and re-runs
     for (int k = tid; k < ne * ne; k += blockDim.x) r0sq[k] = p.r0ab[k] * p.r0ab[k];
-    Atm64Row *rows = scratch + (size_t)blockIdx.x * nrows;
+    Atm64Row *entries = scratch[blockIdx.x].entries;
+    Atm64Scratch::Row *rows = scratch[blockIdx.x].rows;
     const double third = 1.0 / 3.0;
-    // FP32 range test: |d3 - half| <= half in range, but within `slack` of either end of
-    // [0, 2 half] the pair is tested again in FP64. The rounded positions put d3 off by at
-    // most about 5e-7 rc^2.
+    const double rc = sqrt(p.ratm2), cinv = 16.0 / (2.0 * rc);
+    // FP32 range test: |d3 - half| <= half in range, but near either end of [0, 2 half] the
+    // pair is tested again in FP64 (the rounded positions put d3 off by at most about
+    // 5e-7 rc^2). Chunk spheres: distances off by less than 1e-5 rc.
     const float half = (float)(0.5 * p.ratm2 * (1.0 + 1e-5)), sure = half * (1.0f - 4e-5f);
+    const float rcf = (float)rc, slack = 1e-4f * rcf, rc_hi = rcf * rcf * (1.0f + 1e-4f), rc_lo = rcf * rcf * (1.0f - 1e-4f);
     const int cls = lane & 7, member = lane >> 3;
     const unsigned cls_bits = 0x01010101u << cls, below = cls_bits & ((1u << lane) - 1u);
     unsigned long long visits = 0;
@@ -252,42 +346,85 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Row *scra
         if (tid == 0) s_item = atomicAdd(p.work, 1);
         __syncthreads();
         const int S = KIND == ATM64_CENTER ? 1 : p.atmb_split;
-        const int split = s_item % S, unit = s_item / S;
+        const int got = warp_uniform(s_item), split = got % S, unit = got / S;
         const int item = KIND == ATM64_CENTER ? unit : unit * p.shard_world + p.shard_rank;
-        if (item >= (KIND == ATM64_CENTER ? *p.atm_napex : p.n)) break;
+        if (item >= (KIND == ATM64_CENTER ? warp_uniform(*p.atm_napex) : p.n)) break;
         const int a = KIND == ATM64_CENTER ? p.atm_apex[item] : p.sorted_of[p.n - 1 - item];
         const SG &g = p.sg[p.sid[a]];
-        if (KIND != ATM64_CENTER && (g.atm_simple != 0) != (KIND == ATM64_SIMPLE)) continue; // the other instance's
+        if (KIND != ATM64_CENTER && warp_uniform(g.atm_simple) != (KIND == ATM64_SIMPLE ? 1 : 0)) continue; // the other instance's
         const bool ref = KIND == ATM64_WEIGHTED && atm_reference_order(p, g, p.sid[a]);
         const long long e0 = p.atm_off[a];
-        const int m = (int)(p.atm_off[a + 1] - e0);
+        const int m = warp_uniform((int)(p.atm_off[a + 1] - e0));
         const double4 xa = p.xs[a];
         const double *r0a = r0sq + (int)xa.w * ne;
         for (int k = tid; k < ne * NR; k += blockDim.x) yapex[k] = p.Y[(size_t)a * ne * NR + k];
         // types staged together and partner tile: all partners of the apex with as many
-        // types as fit, else one type and the largest tile (one record more is the dummy
-        // partner of idle lanes)
+        // types as fit, else one type and the fewest tiles of equal length
         int types = ne, tile = 0;
         for (;; --types) {
-            tile = min(tile_max, (int)(tile_bytes / atm64_partner_bytes(NR, types) - 1) & ~(ATM64_SEG - 1));
+            tile = min(min(tile_max, 32 * ATM64_CHUNKS),
+                       (int)((tile_bytes - atm64_tile_fixed(NR, types)) / atm64_partner_bytes(NR, types)) & ~31);
             if (types == 1 || tile >= m) break;
         }
-        tile = min(tile, (m + ATM64_SEG - 1) & ~(ATM64_SEG - 1));
+        if (m > 0) {
+            const int tiles = (m + tile - 1) / tile;
+            tile = ((m + tiles - 1) / tiles + 31) & ~31;
+        }
         double2 *sA = reinterpret_cast<double2 *>(area);              // [tile + 1][3]: vx vy | vz id | p g
-        float4 *sF = reinterpret_cast<float4 *>(sA + 3 * (tile + 1)); // [tile + 1]: FP32 position, atom
-        double2 *sR = reinterpret_cast<double2 *>(sF + tile + 1);     // [types][tile + 1][RQ]
+        float4 *sF = reinterpret_cast<float4 *>(sA + 3 * (tile + 1)); // [tile + 32]: FP32 position, atom
+        float4 *sC = sF + tile + 32;                                  // [ATM64_CHUNKS][2]: box of each chunk, sphere radius
+        double2 *sR = reinterpret_cast<double2 *>(sC + 2 * ATM64_CHUNKS); // [types][tile + 1][RQ]
         double acc = 0; // this lane's apex sum (lanes 0..10: energy, dE/dCN, force, virial)
-        for (int b0 = 0; b0 < m; b0 += nrows) {
-            // rows of this split, listed by type
-            const int bn = min(nrows, m - b0);
+        for (int b0 = 0; b0 < m; b0 += ATM64_ROWS) {
+            // set up the entries in Hilbert order (counting sort on a 16^3, 8^3 or 4^3 grid,
+            // whose curves are prefixes of one another) and list this split's rows by type
+            const int bn = min(ATM64_ROWS, m - b0);
+            const int hs = bn >= 1024 ? 0 : (bn >= 128 ? 3 : 6), ncell = ATM64_CELLS >> hs;
+            auto cell_of = [&](const int2 ent) {
+                const double3 v = atm64_pos(p, g, xa, ent, p.xs[ent.x]);
+                const int cx = min(15, max(0, (int)((v.x + rc) * cinv)));
+                const int cy = min(15, max(0, (int)((v.y + rc) * cinv)));
+                const int cz = min(15, max(0, (int)((v.z + rc) * cinv)));
+                return atmb_hilbert(cx, cy, cz) >> hs;
+            };
             __syncthreads();
             for (int k = tid; k <= ne; k += blockDim.x) toff[k] = 0;
+            for (int k = tid; k < ncell; k += blockDim.x) cells[k] = 0;
             __syncthreads();
-            const int first = (split - b0 % S + S) % S; // entries b0 + k with (b0 + k) % S == split
-            for (int k = first + tid * S; k < bn; k += blockDim.x * S) {
-                const Atm64Row r = atm64_entry<NR>(p, g, xa, a, p.atm_ent[e0 + b0 + k], yapex, r0a, true);
-                rows[k] = r;
-                atomicAdd(&toff[r.t + 1], 1);
+            for (int k = tid; k < bn; k += blockDim.x) atomicAdd(&cells[cell_of(p.atm_ent[e0 + b0 + k])], 1);
+            __syncthreads();
+            {
+                // exclusive scan of the cell counts: a run of 32 cells per warp and step
+                const int run = (ncell / 32 + nw - 1) / nw; // steps per warp
+                int carry = 0;
+                for (int r = 0; r < run; ++r) {
+                    const int c = (warp * run + r) * 32 + lane;
+                    const int n = c < ncell ? cells[c] : 0;
+                    int incl = n;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += u;
+                    }
+                    if (c < ncell) cells[c] = carry + incl - n;
+                    carry += __shfl_sync(0xffffffffu, incl, 31);
+                }
+                if (lane == 0) s_tot[warp] = carry;
+                __syncthreads();
+                int before = 0;
+                for (int w = 0; w < warp; ++w) before += s_tot[w];
+                for (int r = 0; r < run; ++r) {
+                    const int c = (warp * run + r) * 32 + lane;
+                    if (c < ncell) cells[c] += before;
+                }
+            }
+            __syncthreads();
+            for (int k = tid; k < bn; k += blockDim.x) {
+                const int2 ent = p.atm_ent[e0 + b0 + k];
+                Atm64Row r = atm64_entry<NR>(p, g, xa, a, ent, yapex, r0a, true);
+                r.k = b0 + k;
+                entries[atomicAdd(&cells[cell_of(ent)], 1)] = r;
+                if (r.k % S == split) atomicAdd(&toff[r.t + 1], 1);
             }
             __syncthreads();
             if (tid == 0)
@@ -296,30 +433,50 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Row *scra
                     toff[t + 1] += toff[t];
                 }
             __syncthreads();
-            for (int k = first + tid * S; k < bn; k += blockDim.x * S)
-                rowperm[atomicAdd(&tpos[rows[k].t], 1)] = (unsigned short)k;
-            __syncthreads();
-            if (toff[ne] == 0) continue; // no row of this split
+            for (int k = tid; k < bn; k += blockDim.x)
+                if (entries[k].k % S == split) {
+                    Atm64Scratch::Row *r = rows + atomicAdd(&tpos[entries[k].t], 1);
+                    r->e = entries[k];
+#pragma unroll
+                    for (int b = 0; b < NR; ++b) {
+                        r->w[b] = p.w[(size_t)entries[k].j * NR + b];
+                        r->dw[b] = p.dw[(size_t)entries[k].j * NR + b];
+                    }
+                }
+            if (warp_uniform(toff[ne]) == 0) continue; // no row of this split
             for (int p0 = 0; p0 < m; p0 += tile) {
-                const int cnt = min(tile, m - p0);
+                const int cnt = min(tile, m - p0), nchunk = (cnt + 31) >> 5;
                 for (int t0 = 0; t0 < ne; t0 += types) {
                     const int tn = min(types, ne - t0);
                     __syncthreads(); // the previous phase is done with the staged data and s_row
-                    const int r1 = toff[t0 + tn];
-                    if (toff[t0] == r1 && !(t0 == 0)) continue;
-                    if (tid == 0) s_row = toff[t0];
+                    const int r0 = warp_uniform(toff[t0]), r1 = warp_uniform(toff[t0 + tn]);
+                    if (r0 == r1 && t0 != 0) continue;
+                    if (tid == 0) s_row = r0;
                     for (int k = tid; k < cnt; k += blockDim.x) {
-                        const int2 ent = p.atm_ent[e0 + p0 + k];
-                        int j = ent.x, tj;
-                        if (t0 == 0) {
-                            const Atm64Row r = atm64_entry<NR>(p, g, xa, a, ent, yapex, r0a, false);
-                            sA[3 * k] = make_double2(r.v[0], r.v[1]);
-                            sA[3 * k + 1] = make_double2(r.v[2], r.id);
-                            sA[3 * k + 2] = make_double2(r.p, r.g);
-                            sF[k] = make_float4((float)r.v[0], (float)r.v[1], (float)r.v[2], __int_as_float(j));
-                            tj = r.t;
+                        int j, tj;
+                        if (m <= ATM64_ROWS) {
+                            const Atm64Row *src = entries + p0 + k;
+                            j = src->j;
+                            tj = src->t;
+                            if (t0 == 0) {
+                                const double2 *q = reinterpret_cast<const double2 *>(src);
+                                const double2 q0 = q[0], q1 = q[1];
+                                sA[3 * k] = q0;
+                                sA[3 * k + 1] = q1;
+                                sA[3 * k + 2] = q[2];
+                                sF[k] = make_float4((float)q0.x, (float)q0.y, (float)q1.x, __int_as_float(j));
+                            }
                         } else {
+                            const int2 ent = p.atm_ent[e0 + p0 + k];
+                            j = ent.x;
                             tj = (int)p.xs[j].w;
+                            if (t0 == 0) {
+                                const Atm64Row r = atm64_entry<NR>(p, g, xa, a, ent, yapex, r0a, false);
+                                sA[3 * k] = make_double2(r.v[0], r.v[1]);
+                                sA[3 * k + 1] = make_double2(r.v[2], r.id);
+                                sA[3 * k + 2] = make_double2(r.p, r.g);
+                                sF[k] = make_float4((float)r.v[0], (float)r.v[1], (float)r.v[2], __int_as_float(j));
+                            }
                         }
                         const double *Y = p.Y + ((size_t)j * ne + t0) * NR;
                         for (int t = 0; t < tn; ++t) {
@@ -332,27 +489,52 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Row *scra
                             for (int b = 0; b < (NR + 1) / 2; ++b) dst[b] = make_double2(q[2 * b], q[2 * b + 1]);
                         }
                     }
-                    // the tail of the last segment lies out of range of every row; the dummy
-                    // partner of idle lanes has p = 0, which makes its terms vanish
-                    for (int k = cnt + tid; k < ((cnt + ATM64_SEG - 1) & ~(ATM64_SEG - 1)); k += blockDim.x) sF[k] = make_float4(3e18f, 3e18f, 3e18f, 0.f);
+                    // far positions after the last partner and at tile .. tile + 31 (out of
+                    // range of every row); the dummy partner's p = 0 makes its terms vanish
+                    if (tid < 32) {
+                        if (cnt + tid < 32 * nchunk) sF[cnt + tid] = make_float4(3e18f, 3e18f, 3e18f, 0.f);
+                        sF[tile + tid] = make_float4(3e18f, 3e18f, 3e18f, __int_as_float(-1));
+                    }
                     if (tid < tn) {
                         if (tid == 0) {
                             sA[3 * tile] = make_double2(3e4, 3e4);
                             sA[3 * tile + 1] = make_double2(3e4, 1.0);
                             sA[3 * tile + 2] = make_double2(0.0, 1.0);
-                            sF[tile] = make_float4(3e18f, 3e18f, 3e18f, __int_as_float(-1));
                         }
                         double2 *dst = sR + ((size_t)tid * (tile + 1) + tile) * RQ;
 #pragma unroll
                         for (int b = 0; b < (NR + 1) / 2; ++b) dst[b] = make_double2(1.0, 1.0);
                     }
                     __syncthreads();
+                    if (t0 == 0) {
+                        // bounding box of each chunk and the radius of its sphere about the box centre
+                        for (int c = warp_uniform(warp); c < nchunk; c += nw) {
+                            const float4 f = sF[min(32 * c + lane, cnt - 1)];
+                            float lo[3] = {f.x, f.y, f.z}, hi[3] = {f.x, f.y, f.z};
+#pragma unroll
+                            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                                for (int q = 0; q < 3; ++q) {
+                                    lo[q] = fminf(lo[q], __shfl_xor_sync(0xffffffffu, lo[q], o));
+                                    hi[q] = fmaxf(hi[q], __shfl_xor_sync(0xffffffffu, hi[q], o));
+                                }
+                            const float cx = 0.5f * (lo[0] + hi[0]), cy = 0.5f * (lo[1] + hi[1]), cz = 0.5f * (lo[2] + hi[2]);
+                            float r2 = (f.x - cx) * (f.x - cx) + (f.y - cy) * (f.y - cy) + (f.z - cz) * (f.z - cz);
+#pragma unroll
+                            for (int o = 16; o > 0; o >>= 1) r2 = fmaxf(r2, __shfl_xor_sync(0xffffffffu, r2, o));
+                            if (lane == 0) {
+                                sC[2 * c] = make_float4(lo[0], lo[1], lo[2], sqrtf(r2));
+                                sC[2 * c + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
+                            }
+                        }
+                        __syncthreads();
+                    }
                     for (;;) {
                         int r = 0;
                         if (lane == 0) r = atomicAdd(&s_row, 1);
-                        r = __shfl_sync(0xffffffffu, r, 0);
+                        r = warp_uniform(r); // (the other lanes hold 0)
                         if (r >= r1) break;
-                        const Atm64Row *X = rows + rowperm[r];
+                        const Atm64Row *X = &rows[r].e;
                         const double vx = X->v[0], vy = X->v[1], vz = X->v[2];
                         const double id1 = X->id, p1 = X->p, h1 = 0.75 * id1;
                         const double g1 = X->g * (6.0 * 4294967296.0 / 43046721.0); // 6 (4/3)^16
@@ -361,146 +543,165 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Row *scra
                         double wx[NR], dwx[NR];
 #pragma unroll
                         for (int b = 0; b < NR; ++b) {
-                            wx[b] = p.w[(size_t)jx * NR + b];
-                            dwx[b] = p.dw[(size_t)jx * NR + b];
+                            wx[b] = rows[r].w[b];
+                            dwx[b] = rows[r].dw[b];
                         }
-                        const float fx = (float)vx, fy = (float)vy, fz = (float)vz;
+                        const float fx = X->f[0], fy = X->f[1], fz = X->f[2];
                         const double2 *sRx = sR + (size_t)(X->t - t0) * RQ * (tile + 1);
                         // sums over this row's visits: w E', w E' lam_xy, wf (f1 + f3),
                         // wf f3 v_y (3), wf f1; v[7] unused
                         double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
                         // weighted kind: (w - wf) (f1 + f3), (w - wf) f3 v_y
                         double dv[4] = {0, 0, 0, 0};
-                        int head = 0, tail = 0; // of this lane's class
-                        for (int c0 = 0; c0 < cnt; c0 += ATM64_SEG) {
-                            // test ATM64_SEG partners, queue those in range
-                            bool in[ATM64_SEG / 32];
-                            bool edge = false;
-                            const float4 *sFc = sF + c0 + lane;
-#pragma unroll
-                            for (int c = 0; c < ATM64_SEG / 32; ++c) {
-                                const float4 f = sFc[32 * c];
-                                const float dx = fx - f.x, dy = fy - f.y, dz = fz - f.z;
-                                const float off = fabsf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) - half);
-                                in[c] = off <= half;
-                                edge |= in[c] & (off >= sure);
+                        // one visit per lane, of partner k
+                        auto visit = [&](int k) {
+                            Atm64Visit V;
+                            atm64_visit<NR>(vx, vy, vz, d1, id1, h1, p1, g1, wx, dwx, sA + 3 * k, sRx + RQ * k, V);
+                            if (KIND == ATM64_WEIGHTED) {
+                                const int jy = __float_as_int(sF[k].w);
+                                if (jx == jy || jx == a || jy == a) {
+                                    double w, wf;
+                                    atm_weights(jx == jy, jx == a, jy == a, ref, p.atm_force_scaled != 0, w, wf);
+                                    const double d3w = (w - wf) * V.f3;
+                                    dv[0] = fma(w - wf, V.f1 + V.f3, dv[0]);
+                                    dv[1] = fma(d3w, V.vx, dv[1]);
+                                    dv[2] = fma(d3w, V.vy, dv[2]);
+                                    dv[3] = fma(d3w, V.vz, dv[3]);
+                                    V.E *= w;
+                                    V.f1 *= wf;
+                                    V.f3 *= wf;
+                                }
                             }
-                            if (__any_sync(0xffffffffu, edge)) {
+                            v[0] += V.E;
+                            v[1] = fma(V.E, V.lam, v[1]);
+                            v[2] += V.f1 + V.f3;
+                            v[3] = fma(V.f3, V.vx, v[3]);
+                            v[4] = fma(V.f3, V.vy, v[4]);
+                            v[5] = fma(V.f3, V.vz, v[5]);
+                            v[6] += V.f1;
+                        };
+                        // classify the chunks (lane l: chunks l and l + 32) and list them. A
+                        // chunk is all in range only when it is whole and x lies outside its
+                        // box (no pair closer than 0.1 bohr)
+                        int nfull = 0, nmixed = 0;
+                        __syncwarp();
 #pragma unroll
-                                for (int c = 0; c < ATM64_SEG / 32; ++c)
-                                    if (in[c]) {
-                                        const double2 *A = sA + 3 * (c0 + 32 * c + lane);
+                        for (int h = 0; h < ATM64_CHUNKS / 32; ++h) {
+                            const int c = 32 * h + lane;
+                            bool none = true, all = false;
+                            if (c < nchunk) {
+                                // nearest and farthest points of its box, its sphere
+                                const float4 L = sC[2 * c], H = sC[2 * c + 1];
+                                const float ax = fx - L.x, bx = H.x - fx, ay = fy - L.y, by = H.y - fy, az = fz - L.z, bz = H.z - fz;
+                                const float nx = fmaxf(0.f, -fminf(ax, bx)), ny = fmaxf(0.f, -fminf(ay, by)), nz = fmaxf(0.f, -fminf(az, bz));
+                                const float gx = fmaxf(ax, bx), gy = fmaxf(ay, by), gz = fmaxf(az, bz);
+                                const float near2 = nx * nx + ny * ny + nz * nz, far2 = gx * gx + gy * gy + gz * gz;
+                                const float d2 = 0.25f * ((ax - bx) * (ax - bx) + (ay - by) * (ay - by) + (az - bz) * (az - bz));
+                                const float past = rcf + L.w + slack, inside = fmaxf(0.f, rcf - L.w - slack);
+                                none = near2 > rc_hi || d2 > past * past;
+                                all = (far2 < rc_lo || d2 < inside * inside) && near2 > 0.01f && 32 * c + 32 <= cnt;
+                            }
+                            const unsigned fb = __ballot_sync(0xffffffffu, all), mb = __ballot_sync(0xffffffffu, !all && !none);
+                            const unsigned lt = (1u << lane) - 1u;
+                            if (all) list[nfull + __popc(fb & lt)] = (unsigned short)(32 * c);
+                            if (!all && !none) list[ATM64_LIST - 1 - (nmixed + __popc(mb & lt))] = (unsigned short)(32 * c);
+                            nfull = warp_uniform(nfull + __popc(fb));
+                            nmixed = warp_uniform(nmixed + __popc(mb));
+                        }
+                        // (the mixed list is filled up with the far positions)
+                        if (lane < ATM64_SEG - 1 && nmixed + lane < ((nmixed + ATM64_SEG - 1) & ~(ATM64_SEG - 1)))
+                            list[ATM64_LIST - 1 - (nmixed + lane)] = (unsigned short)tile;
+                        __syncwarp();
+                        if (lane == 0) visits += 32 * nfull;
+#pragma unroll 1
+                        for (int i = 0; i < nfull; ++i) visit(list[i] + lane);
+#pragma unroll 1
+                        for (int i0 = 0; i0 < nmixed; i0 += ATM64_GROUP) {
+                            // test the partners of up to ATM64_GROUP mixed chunks, queue those
+                            // in range (k / 8: the class is k mod 8)
+                            const int i1 = min(nmixed, i0 + ATM64_GROUP);
+                            int tail = 0; // queued partners of this lane's class
+                            __syncwarp();
+#pragma unroll 1
+                            for (int i = i0; i < i1; i += ATM64_SEG) {
+                                unsigned bits[ATM64_SEG];
+                                int k[ATM64_SEG];
+                                bool edge = false;
+#pragma unroll
+                                for (int c = 0; c < ATM64_SEG; ++c) {
+                                    k[c] = list[ATM64_LIST - 1 - (i + c)] + lane;
+                                    const float4 f = sF[k[c]];
+                                    const float dx = fx - f.x, dy = fy - f.y, dz = fz - f.z;
+                                    const float off = fabsf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) - half);
+                                    bits[c] = __ballot_sync(0xffffffffu, off <= half);
+                                    edge |= off <= half && off >= sure;
+                                }
+                                if (warp_uniform(edge ? 1 : 0)) {
+#pragma unroll
+                                    for (int c = 0; c < ATM64_SEG; ++c) {
+                                        const double2 *A = sA + 3 * min(k[c], tile);
                                         const double rx = vx - A[0].x, ry = vy - A[0].y, rz = vz - A[1].x;
                                         const double d3 = fma(rx, rx, fma(ry, ry, rz * rz));
-                                        in[c] = d3 <= p.ratm2 && d3 >= 1e-12; // also drops x == y
-                                    }
-                            }
-#pragma unroll
-                            for (int c = 0; c < ATM64_SEG / 32; ++c) {
-                                const unsigned bits = __ballot_sync(0xffffffffu, in[c]);
-                                const int slot = ((tail + __popc(bits & below)) & (ATM64_QCAP - 1)) * 8 + cls;
-                                if (in[c]) queue[slot] = (unsigned short)(c0 + 32 * c + lane);
-                                tail += __popc(bits & cls_bits);
-                            }
-                            __syncwarp();
-                            // two visits per lane while all lanes are busy (after the last
-                            // partners: while any is), and while a class could overflow next
-                            const int least = c0 + ATM64_SEG >= cnt ? 0 : 8;
-                            for (;;) {
-                                const int pend = tail - head;
-                                if (least ? !(__all_sync(0xffffffffu, pend >= 8) ||
-                                              __any_sync(0xffffffffu, pend > ATM64_QCAP - ATM64_SEG / 8))
-                                          : !__any_sync(0xffffffffu, pend > 0))
-                                    break;
-                                int k[2];
-                                Atm64Visit V[2];
-#pragma unroll
-                                for (int h = 0; h < 2; ++h) {
-                                    const int i = head + member + 4 * h;
-                                    k[h] = queue[(i & (ATM64_QCAP - 1)) * 8 + cls];
-                                    k[h] = i < tail ? k[h] : tile;
-                                }
-                                head = min(head + 8, tail);
-#pragma unroll
-                                for (int h = 0; h < 2; ++h)
-                                    atm64_visit<NR>(vx, vy, vz, d1, id1, h1, p1, g1, wx, dwx, sA + 3 * k[h], sRx + RQ * k[h], V[h]);
-                                if (KIND == ATM64_WEIGHTED) {
-                                    const int jy[2] = {__float_as_int(sF[k[0]].w), __float_as_int(sF[k[1]].w)};
-                                    if (jx == jy[0] || jx == jy[1] || jx == a || jy[0] == a || jy[1] == a) {
-#pragma unroll
-                                        for (int h = 0; h < 2; ++h) {
-                                            double w, wf;
-                                            atm_weights(jx == jy[h], jx == a, jy[h] == a, ref, p.atm_force_scaled != 0, w, wf);
-                                            const double d3w = (w - wf) * V[h].f3;
-                                            const double2 *A = sA + 3 * k[h];
-                                            dv[0] = fma(w - wf, V[h].f1 + V[h].f3, dv[0]);
-                                            dv[1] = fma(d3w, A[0].x, dv[1]);
-                                            dv[2] = fma(d3w, A[0].y, dv[2]);
-                                            dv[3] = fma(d3w, A[1].x, dv[3]);
-                                            V[h].E *= w;
-                                            V[h].f1 *= wf;
-                                            V[h].f3 *= wf;
-                                        }
+                                        bits[c] &= __ballot_sync(0xffffffffu, d3 <= p.ratm2 && d3 >= 1e-12); // also drops x == y
                                     }
                                 }
 #pragma unroll
-                                for (int h = 0; h < 2; ++h) {
-                                    v[0] += V[h].E;
-                                    v[1] = fma(V[h].E, V[h].lam, v[1]);
-                                    v[2] += V[h].f1 + V[h].f3;
-                                    v[3] = fma(V[h].f3, V[h].vx, v[3]);
-                                    v[4] = fma(V[h].f3, V[h].vy, v[4]);
-                                    v[5] = fma(V[h].f3, V[h].vz, v[5]);
-                                    v[6] += V[h].f1;
+                                for (int c = 0; c < ATM64_SEG; ++c) {
+                                    if (bits[c] & (1u << lane))
+                                        queue[(tail + __popc(bits[c] & below)) * 8 + cls] = (unsigned char)(k[c] >> 3);
+                                    tail += __popc(bits[c] & cls_bits);
                                 }
                             }
                             __syncwarp();
+                            const int rounds = warp_uniform((tail + 3) >> 2);
+#pragma unroll 1
+                            for (int i = 0; i < rounds; ++i) {
+                                const int q = 4 * i + member;
+                                int k = queue[q * 8 + cls] * 8 + cls;
+                                k = q < tail ? k : tile;
+                                visit(k);
+                            }
+                            if (member == 0) visits += (unsigned)tail;
                         }
-                        if (member == 0) visits += (unsigned)tail;
                         if (KIND == ATM64_CENTER) {
 #pragma unroll
                             for (int k = 0; k < 7; ++k) v[k] *= third;
                         }
-                        // the row's sums: entry shares (atomics by lanes 11..15) and apex sums
+                        // the row's sums; then each of 16 lanes forms one output from them (rule
+                        // and coefficients in s_rule, s_coef): lanes 0..10 apex sums, 11..15
+                        // the entry's energy, dE/dCN and force
                         const double tot = atm64_reduce8(v);
-                        const double SE = -__shfl_sync(0xffffffffu, tot, atm64_lane(0));
-                        const double SD = -__shfl_sync(0xffffffffu, tot, atm64_lane(1));
-                        const double SF = __shfl_sync(0xffffffffu, tot, atm64_lane(2));
-                        const double Wx = __shfl_sync(0xffffffffu, tot, atm64_lane(3));
-                        const double Wy = __shfl_sync(0xffffffffu, tot, atm64_lane(4));
-                        const double Wz = __shfl_sync(0xffffffffu, tot, atm64_lane(5));
-                        const double SA = __shfl_sync(0xffffffffu, tot, atm64_lane(6));
-                        double Sv = SF, Ux = Wx, Uy = Wy, Uz = Wz; // virial sums (weights w)
-                        if (KIND == ATM64_WEIGHTED && __any_sync(0xffffffffu, dv[0] != 0.0 || dv[1] != 0.0 || dv[2] != 0.0 || dv[3] != 0.0)) {
-                            Sv += warp_sum(dv[0]);
-                            Ux += warp_sum(dv[1]);
-                            Uy += warp_sum(dv[2]);
-                            Uz += warp_sum(dv[3]);
+                        if ((lane & 3) == 0) sr[((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = tot;
+                        if (lane == 1) {
+                            sr[ATM64_SV] = vx;
+                            sr[ATM64_SV + 1] = vy;
+                            sr[ATM64_SV + 2] = vz;
+                            sr[ATM64_SAE] = X->lam_ae;
+                            sr[ATM64_SEA] = X->lam_ea;
                         }
-                        // component of each lane: force lanes 2..4 and 13..15, virial lanes
-                        // 5..10 (xx yy zz xy xz yz)
-                        const int ca = lane < 5 ? lane - 2 : (lane < 8 ? lane - 5 : (lane < 10 ? 0 : (lane == 10 ? 1 : lane - 13)));
-                        const int cb = lane < 8 ? ca : (lane == 8 ? 1 : 2);
-                        const double va = ca == 0 ? vx : (ca == 1 ? vy : vz), vb = cb == 0 ? vx : (cb == 1 ? vy : vz);
-                        const double Ua = ca == 0 ? Ux : (ca == 1 ? Uy : Uz), Ub = cb == 0 ? Ux : (cb == 1 ? Uy : Uz);
-                        const double Wa = ca == 0 ? Wx : (ca == 1 ? Wy : Wz);
-                        // apex: energy E/3 per pair and dE/dCN E/2 lam over both visits of a
-                        // pair, force -f1 v_x per visit, virial f r (x) r with the x-y side's
-                        // cross part split evenly between the two visits
-                        if (lane == 0)
-                            acc += SE * (0.5 * third);
-                        else if (lane == 1)
-                            acc += 0.5 * X->lam_ae * SE;
-                        else if (lane < 5)
-                            acc -= SA * va;
-                        else if (lane < 11)
-                            acc += Sv * va * vb - 0.5 * (Ua * vb + Ub * va);
-                        else if (lane == 11)
-                            atomicAdd(&p.eb[jx], SE * third);
-                        else if (lane == 12)
-                            atomicAdd(&p.gb[jx], 0.5 * (X->lam_ea * SE + SD));
-                        else if (lane < 16)
-                            atomicAdd(&p.fb[3 * jx + ca], SF * va - Wa);
+                        __syncwarp();
+                        if (KIND == ATM64_WEIGHTED) {
+                            // virial sums (weights w)
+                            double d[4] = {0, 0, 0, 0};
+                            if (warp_uniform(dv[0] != 0.0 || dv[1] != 0.0 || dv[2] != 0.0 || dv[3] != 0.0))
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) d[k] = warp_sum(dv[k]);
+                            if (lane == 0)
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) sr[ATM64_SVIR + k] = sr[2 + k] + d[k];
+                            __syncwarp();
+                        }
+                        if (lane < 16) {
+                            const unsigned long long rule = s_rule[lane];
+                            auto at = [&](int q) { return sr[(rule >> (8 * q)) & 0xff]; };
+                            const double va = at(1), vb = at(2);
+                            const double val = s_coef[lane][0] * at(5) * sr[0] + s_coef[lane][1] * sr[1] +
+                                               s_coef[lane][2] * at(0) * va * vb - s_coef[lane][3] * (at(3) * vb + at(4) * va);
+                            if (lane < 11)
+                                acc += val;
+                            else
+                                atomicAdd(lane == 11 ? p.eb + jx : (lane == 12 ? p.gb + jx : p.fb + 3 * (size_t)jx + (lane - 13)), val);
+                        }
                     }
                 }
             }

@@ -1007,9 +1007,9 @@ __global__ void k_chain32(KP p, const double *Gd) {
 }
 
 #include "d3_pairs.cuh"
-#include "d3_atm.cuh"
 #include "d3_atm32.cuh"
 #include "d3_atm32b.cuh"
+#include "d3_atm.cuh"
 #include "d3_surrogate.cuh"
 
 // ------------------------------------------------------------------------------------
@@ -1272,7 +1272,7 @@ struct Engine {
     DBuf<float4> xs32;
     DBuf<float> w32, dw32, Y32, YD32;
     DBuf<float4> atmb_scratch;
-    DBuf<Atm64Row> atm64_scratch;
+    DBuf<Atm64Scratch> atm64_scratch;
     DBuf<long long> atm_off;
     DBuf<int2> atm_ent;
     long long atm_cap = 0;
@@ -1912,16 +1912,15 @@ static int apex_split(long long apexes, long long ctas, int most, double setup) 
 
 // CTAs per SM of the FP64 ATM kernel, their shared memory and the splits of an apex
 struct Atm64Shape {
-    int ctas, nrows, split;
+    int ctas, split;
     size_t fixed, tile_bytes;
 };
 static Atm64Shape atm64_shape(const Engine *e, int world) {
     Atm64Shape sh;
     const int want = e->opt.atm_ctas_per_sm;
     sh.ctas = want <= 0 ? 1 : (want >= 4 ? 4 : (want >= 2 ? 2 : 1));
-    sh.nrows = ATM64_ROWS / sh.ctas;
     const size_t limit = std::min<size_t>(227 * 1024, 228 * 1024 / sh.ctas - 1024) - ATM64_STATIC;
-    sh.fixed = atm64_fixed_bytes(e->ne, e->nref, ATM64_THREADS / 32 / sh.ctas, sh.nrows);
+    sh.fixed = atm64_fixed_bytes(e->ne, e->nref, ATM64_THREADS / 32 / sh.ctas);
     sh.tile_bytes = limit - sh.fixed;
     sh.split = apex_split(std::max<long long>(1, (long long)e->n / std::max(1, world)), e->dev_sms * sh.ctas, 32, 0.01);
     return sh;
@@ -1985,7 +1984,7 @@ static KP make_kp(Engine *e) {
     }
     if (e->use_atm && !p.precision) {
         const Atm64Shape sh = atm64_shape(e, 1);
-        e->atm64_scratch.ensure((size_t)e->dev_sms * sh.ctas * sh.nrows);
+        e->atm64_scratch.ensure((size_t)e->dev_sms * sh.ctas);
     }
     p.atm_force_scaled = e->opt.atm_force_scaled ? 1 : 0;
     p.anyshift = e->anyshift.p;
@@ -2099,8 +2098,8 @@ static void launch_atm64(Engine *e, const KP &p0, cudaStream_t s, bool center) {
         if (!kind[k]) continue;
         if (k == ATM64_WEIGHTED && kind[ATM64_SIMPLE]) D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
         atm_occupancy(e, cache[k], sm, fns[k]);
-        int nrows = sh.nrows, tile_bytes = (int)sh.tile_bytes, tmax = tile_max;
-        void *args[] = {(void *)&p, (void *)&e->atm64_scratch.p, &nrows, &tile_bytes, &tmax};
+        int tile_bytes = (int)sh.tile_bytes, tmax = tile_max;
+        void *args[] = {(void *)&p, (void *)&e->atm64_scratch.p, &tile_bytes, &tmax};
         D3_CUDA(cudaLaunchKernel(fns[k], dim3(grid), dim3(ATM64_THREADS / sh.ctas), args, sm, s));
     }
 }
