@@ -1637,48 +1637,41 @@ static void build_structures(Engine *e, int nstruct, const uint64_t *counts, con
         r.atom_base = atom_base;
         r.natoms = (int)counts[k];
         atom_base += (int)counts[k];
-        auto add = [&](double rc, int &off, int &cnt) {
-            auto st = build_stencil(g, r.nb, rc);
-            off = (int)rows.size();
-            cnt = (int)st.size();
-            for (auto &x : st) rows.push_back(make_int4(x.dy, x.dz, x.dxlo, x.dxhi));
-        };
-        add(e->rc, r.st2_off, r.st2_n);
-        add(e->rc_cn, r.stc_off, r.stc_n);
-        if (e->use_atm) add(e->rc_atm, r.sta_off, r.sta_n);
         // two-body atom groups: blocks of gy x gz bin rows holding about 16 atoms per
         // column, so that a group of 32 spans one or two columns
-        {
-            const double per_bin = (double)counts[k] / std::max(1, r.nbins);
-            const int gb = std::max(1, std::min(4, (int)std::lround(std::sqrt(16.0 / std::max(per_bin, 1e-3)))));
-            const int gy = std::min(gb, r.nb[1]), gz = std::min(gb, r.nb[2]);
-            std::vector<StencilRow> s2;
-            for (int q = r.st2_off; q < r.st2_off + r.st2_n; ++q)
-                s2.push_back({rows[q].x, rows[q].y, rows[q].z, rows[q].w});
-            const auto blk = merge_block_stencil(s2, gy, gz);
-            r.st2b_off = (int)rows.size();
-            r.st2b_n = (int)blk.size();
-            for (auto &x : blk) rows.push_back(make_int4(x.dy, x.dz, x.dxlo, x.dxhi));
-            std::vector<StencilRow> sc;
-            for (int q = r.stc_off; q < r.stc_off + r.stc_n; ++q)
-                sc.push_back({rows[q].x, rows[q].y, rows[q].z, rows[q].w});
-            const auto blkc = merge_block_stencil(sc, gy, gz);
-            r.stcb_off = (int)rows.size();
-            r.stcb_n = (int)blkc.size();
-            for (auto &x : blkc) rows.push_back(make_int4(x.dy, x.dz, x.dxlo, x.dxhi));
-            if (e->use_atm) {
-                std::vector<StencilRow> sa;
-                for (int q = r.sta_off; q < r.sta_off + r.sta_n; ++q)
-                    sa.push_back({rows[q].x, rows[q].y, rows[q].z, rows[q].w});
-                const auto blka = merge_block_stencil(sa, gy, gz);
-                r.stab_off = (int)rows.size();
-                r.stab_n = (int)blka.size();
-                for (auto &x : blka) rows.push_back(make_int4(x.dy, x.dz, x.dxlo, x.dxhi));
+        const double per_bin = (double)counts[k] / std::max(1, r.nbins);
+        const int gb = std::max(1, std::min(4, (int)std::lround(std::sqrt(16.0 / std::max(per_bin, 1e-3)))));
+        const int gy = std::min(gb, r.nb[1]), gz = std::min(gb, r.nb[2]);
+        // stencils of a bin and of a block for each cutoff (equal cutoffs share one)
+        struct Cut {
+            double rc;
+            int *off, *cnt, *boff, *bcnt;
+        } cuts[3] = {{e->rc, &r.st2_off, &r.st2_n, &r.st2b_off, &r.st2b_n},
+                     {e->rc_cn, &r.stc_off, &r.stc_n, &r.stcb_off, &r.stcb_n},
+                     {e->rc_atm, &r.sta_off, &r.sta_n, &r.stab_off, &r.stab_n}};
+        const int ncut = e->use_atm ? 3 : 2;
+        auto add = [&](const std::vector<StencilRow> &st, int *off, int *cnt) {
+            *off = (int)rows.size();
+            *cnt = (int)st.size();
+            for (const StencilRow &x : st) rows.push_back(make_int4(x.dy, x.dz, x.dxlo, x.dxhi));
+        };
+        for (int c = 0; c < ncut; ++c) {
+            int q = 0;
+            while (q < c && cuts[q].rc != cuts[c].rc) ++q;
+            if (q < c) {
+                *cuts[c].off = *cuts[q].off;
+                *cuts[c].cnt = *cuts[q].cnt;
+                *cuts[c].boff = *cuts[q].boff;
+                *cuts[c].bcnt = *cuts[q].bcnt;
+                continue;
             }
-            for (int bz = 0; bz < r.nb[2]; bz += gz)
-                for (int by = 0; by < r.nb[1]; by += gy)
-                    srow.push_back(make_int4(k, by, bz, std::min(gy, r.nb[1] - by) | (std::min(gz, r.nb[2] - bz) << 8)));
+            const auto st = build_stencil(g, r.nb, cuts[c].rc);
+            add(st, cuts[c].off, cuts[c].cnt);
+            add(merge_block_stencil(st, gy, gz), cuts[c].boff, cuts[c].bcnt);
         }
+        for (int bz = 0; bz < r.nb[2]; bz += gz)
+            for (int by = 0; by < r.nb[1]; by += gy)
+                srow.push_back(make_int4(k, by, bz, std::min(gy, r.nb[1] - by) | (std::min(gz, r.nb[2] - bz) << 8)));
         sid.insert(sid.end(), counts[k], k);
     }
     e->sg = sg;

@@ -1,11 +1,9 @@
-#include <map>
 // Host-side cell geometry (see d3_geometry.h).
 #include "d3_geometry.h"
 
 #include <algorithm>
 #include <cmath>
 #include <limits>
-#include <map>
 
 namespace d3 {
 
@@ -81,66 +79,58 @@ void choose_bins(const CellGeom &g, double target, int64_t max_bins, int nb[3]) 
 
 namespace {
 
-// min over u in [-1,1]^3 of (d+u)^T G (d+u): exact, by enumerating which coordinates
-// sit on a bound (27 active sets) and solving the free ones.
-double min_dist2(const double G[3][3], const double d[3]) {
-    double best = std::numeric_limits<double>::infinity();
-    for (int code = 0; code < 27; ++code) {
-        int st[3] = {code % 3, (code / 3) % 3, code / 9}; // 0 free, 1 lower, 2 upper
-        double v[3];
-        int fr[3], nf = 0;
-        for (int k = 0; k < 3; ++k) {
-            if (st[k] == 1)
-                v[k] = d[k] - 1.0;
-            else if (st[k] == 2)
-                v[k] = d[k] + 1.0;
-            else {
-                v[k] = 0.0;
-                fr[nf++] = k;
-            }
-        }
-        // solve G_ff x_f = -G_fc v_c  (x_f = d_f + u_f)
-        double rhs[3], A[3][3];
-        for (int a = 0; a < nf; ++a) {
-            rhs[a] = 0;
-            for (int k = 0; k < 3; ++k)
-                if (st[k] != 0) rhs[a] -= G[fr[a]][k] * v[k];
-            for (int b = 0; b < nf; ++b) A[a][b] = G[fr[a]][fr[b]];
-        }
-        double x[3] = {0, 0, 0};
-        bool ok = true;
-        if (nf == 1) {
-            x[0] = rhs[0] / A[0][0];
-        } else if (nf == 2) {
-            double det = A[0][0] * A[1][1] - A[0][1] * A[1][0];
-            if (std::fabs(det) < 1e-300) ok = false;
-            else {
-                x[0] = (rhs[0] * A[1][1] - A[0][1] * rhs[1]) / det;
-                x[1] = (A[0][0] * rhs[1] - rhs[0] * A[1][0]) / det;
-            }
-        } else if (nf == 3) {
-            x[0] = x[1] = x[2] = 0.0; // unconstrained minimum of a PD form is the origin
-        }
-        if (!ok) continue;
-        for (int a = 0; a < nf; ++a) {
-            double u = x[a] - d[fr[a]];
-            if (u < -1.0 || u > 1.0) {
-                ok = false;
-                break;
-            }
-            v[fr[a]] = x[a];
-        }
-        if (!ok) continue;
-        double q = 0;
+// Largest v_x with v^T G v <= r2 over y0 <= v_y <= y1, z0 <= v_z <= z1 (-inf when there is
+// none). v_x over the ellipsoid is concave in (v_y, v_z), so the maximum is the ellipsoid's
+// own one when it lies in the box, else the largest of the edges' stationary points that
+// lie on their edge and of the corners.
+struct RowExtent {
+    double G[3][3], r2;
+    double xs, ys, zs; // point of the ellipsoid with the largest v_x
+    RowExtent(const double g[3][3], double rr2) : r2(rr2) {
         for (int a = 0; a < 3; ++a)
-            for (int b = 0; b < 3; ++b) q += v[a] * G[a][b] * v[b];
-        best = std::min(best, q);
+            for (int b = 0; b < 3; ++b) G[a][b] = g[a][b];
+        // G^-1 e_x up to the common factor 1 / det
+        const double c0 = G[1][1] * G[2][2] - G[1][2] * G[1][2], c1 = G[0][2] * G[1][2] - G[0][1] * G[2][2],
+                     c2 = G[0][1] * G[1][2] - G[0][2] * G[1][1];
+        const double det = G[0][0] * c0 + G[0][1] * c1 + G[0][2] * c2;
+        const double f = std::sqrt(r2 / (det * c0));
+        xs = f * c0;
+        ys = f * c1;
+        zs = f * c2;
     }
-    return best;
-}
+    // v_y = c (a = 1, b = 2) or v_z = c (a = 2, b = 1) fixed, the other one in [lo, hi]
+    double edge(int a, int b, double c, double lo, double hi) const {
+        const double ib = 1.0 / G[b][b], k = G[0][b] * ib;
+        const double A = G[0][0] - G[0][b] * k, B = c * (G[0][a] - G[a][b] * k), C = c * c * (G[a][a] - G[a][b] * G[a][b] * ib) - r2;
+        const double D = B * B - A * C;
+        if (D < 0.0) return -std::numeric_limits<double>::infinity();
+        const double x = (-B + std::sqrt(D)) / A, w = -(G[0][b] * x + G[a][b] * c) * ib;
+        return w >= lo && w <= hi ? x : -std::numeric_limits<double>::infinity();
+    }
+    double corner(double y, double z) const {
+        const double B = G[0][1] * y + G[0][2] * z;
+        const double C = G[1][1] * y * y + 2.0 * G[1][2] * y * z + G[2][2] * z * z - r2;
+        const double D = B * B - G[0][0] * C;
+        return D < 0.0 ? -std::numeric_limits<double>::infinity() : (-B + std::sqrt(D)) / G[0][0];
+    }
+    double largest(double y0, double y1, double z0, double z1) const {
+        if (ys >= y0 && ys <= y1 && zs >= z0 && zs <= z1) return xs;
+        double x = std::max(std::max(edge(1, 2, y0, z0, z1), edge(1, 2, y1, z0, z1)),
+                            std::max(edge(2, 1, z0, y0, y1), edge(2, 1, z1, y0, y1)));
+        x = std::max(x, std::max(std::max(corner(y0, z0), corner(y0, z1)), std::max(corner(y1, z0), corner(y1, z1))));
+        return x;
+    }
+};
 
 } // namespace
 
+// A bin offset d belongs to the stencil when some v in d + [-1, 1]^3 (bin units) has
+// v^T G v <= r^2. For a row (dy, dz) these dx are the integers within 1 of the v_x range of
+// the ellipsoid over the row's box, and by inversion the smallest v_x of a row is minus the
+// largest one of the row (-dy, -dz): one closed-form maximum per row. (Testing every bin of
+// every row with a 27-case quadratic program took 1.4 ms for a 10-atom box, 11 ms for the
+// 20,000-atom box and 289 ms for 48 small structures per set_cell; now 0.05, 0.13 and 1.8 ms
+// for the whole call.)
 std::vector<StencilRow> build_stencil(const CellGeom &g, const int nb[3], double r) {
     double M[3][3];
     for (int k = 0; k < 3; ++k)
@@ -149,42 +139,53 @@ std::vector<StencilRow> build_stencil(const CellGeom &g, const int nb[3], double
     for (int a = 0; a < 3; ++a)
         for (int b = 0; b < 3; ++b) G[a][b] = M[a][0] * M[b][0] + M[a][1] * M[b][1] + M[a][2] * M[b][2];
     const double rr = r * (1.0 + 1e-9) + 1e-6;
-    const double r2 = rr * rr;
     int ext[3];
     for (int k = 0; k < 3; ++k) ext[k] = (int)std::ceil(rr / (g.height[k] / nb[k])) + 1;
+    const RowExtent E(G, rr * rr);
+    const int ny = 2 * ext[1] + 1, nz = 2 * ext[2] + 1;
+    std::vector<double> top((size_t)ny * nz);
+    for (int dz = -ext[2]; dz <= ext[2]; ++dz)
+        for (int dy = -ext[1]; dy <= ext[1]; ++dy)
+            top[(size_t)(dz + ext[2]) * ny + dy + ext[1]] = E.largest(dy - 1.0, dy + 1.0, dz - 1.0, dz + 1.0);
     std::vector<StencilRow> rows;
+    rows.reserve(top.size());
     for (int dz = -ext[2]; dz <= ext[2]; ++dz)
         for (int dy = -ext[1]; dy <= ext[1]; ++dy) {
-            int lo = 1, hi = 0;
-            for (int dx = -ext[0]; dx <= ext[0]; ++dx) {
-                double d[3] = {(double)dx, (double)dy, (double)dz};
-                if (min_dist2(G, d) <= r2) {
-                    if (lo > hi) lo = hi = dx;
-                    else hi = dx;
-                }
-            }
-            if (lo <= hi) rows.push_back({dy, dz, lo, hi});
+            const double hi = top[(size_t)(dz + ext[2]) * ny + dy + ext[1]];
+            const double lo = -top[(size_t)(ext[2] - dz) * ny + ext[1] - dy];
+            if (!std::isfinite(hi) || !std::isfinite(lo)) continue;
+            const int a = (int)std::ceil(lo - 1.0 - 1e-9), b = (int)std::floor(hi + 1.0 + 1e-9);
+            if (a <= b) rows.push_back({dy, dz, a, b});
         }
     return rows;
 }
 
 std::vector<StencilRow> merge_block_stencil(const std::vector<StencilRow> &st, int gy, int gz) {
-    std::map<std::pair<int, int>, std::pair<int, int>> m; // (dz, dy) -> (lo, hi)
+    if (st.empty()) return {};
+    int y0 = st[0].dy, y1 = y0, z0 = st[0].dz, z1 = z0;
+    for (const StencilRow &r : st) {
+        y0 = std::min(y0, r.dy);
+        y1 = std::max(y1, r.dy);
+        z0 = std::min(z0, r.dz);
+        z1 = std::max(z1, r.dz);
+    }
+    const int ny = y1 - y0 + gy, nz = z1 - z0 + gz;
+    std::vector<StencilRow> all((size_t)ny * nz, StencilRow{0, 0, 1, 0}); // (empty: dxlo > dxhi)
     for (int oz = 0; oz < gz; ++oz)
         for (int oy = 0; oy < gy; ++oy)
             for (const StencilRow &r : st) {
-                const auto key = std::make_pair(r.dz + oz, r.dy + oy);
-                auto it = m.find(key);
-                if (it == m.end())
-                    m.emplace(key, std::make_pair(r.dxlo, r.dxhi));
+                StencilRow &q = all[(size_t)(r.dz + oz - z0) * ny + r.dy + oy - y0];
+                if (q.dxlo > q.dxhi)
+                    q = {r.dy + oy, r.dz + oz, r.dxlo, r.dxhi};
                 else {
-                    it->second.first = std::min(it->second.first, r.dxlo);
-                    it->second.second = std::max(it->second.second, r.dxhi);
+                    q.dxlo = std::min(q.dxlo, r.dxlo);
+                    q.dxhi = std::max(q.dxhi, r.dxhi);
                 }
             }
-    std::vector<StencilRow> out;
-    out.reserve(m.size());
-    for (const auto &kv : m) out.push_back({kv.first.second, kv.first.first, kv.second.first, kv.second.second});
+    std::vector<StencilRow> out; // ordered by dz, then dy
+    out.reserve(all.size());
+    for (const StencilRow &r : all)
+        if (r.dxlo <= r.dxhi) out.push_back(r);
     return out;
 }
 

@@ -32,7 +32,7 @@ bool reference_box(const float cell_f[9], float rc, float rc_cn, int64_t mcb[3])
 void choose_bins(const CellGeom &g, double target_width, int64_t max_bins, int nb[3]);
 
 // All bin offsets whose closest possible point pair is within r (+ margin),
-// compressed into x-rows. Exact convex-QP distance between parallelepiped bins.
+// compressed into x-rows (exact for parallelepiped bins; ordered by dz, then dy).
 std::vector<StencilRow> build_stencil(const CellGeom &g, const int nb[3], double r);
 
 // Stencil of a block of gy x gz bin rows (offsets relative to the block's first row): for
