@@ -149,7 +149,8 @@ struct KP {
     int nsrow;
     int4 *groups;
     int *gcount;             // groups cut this evaluation (the passes' work counters follow)
-    int gslices;
+    int gslices; // of the pass at hand
+    int gslices_of[3]; // two-body, CN and chain rule, ATM lists
     double *gpart;
 };
 
@@ -1006,6 +1007,7 @@ __global__ void k_chain32(KP p, const double *Gd) {
     }
 }
 
+#include "d3_roots.cuh"
 #include "d3_pairs.cuh"
 #include "d3_atm32.cuh"
 #include "d3_atm32b.cuh"
@@ -1989,12 +1991,25 @@ static KP make_kp(Engine *e) {
     p.gslices = 0;
     p.gpart = nullptr;
     if (pairs_grouped(e)) {
-        // slices per group: about six work items per resident warp, so that the items
-        // taken last are short against the pass
-        const int warps = e->dev_sms * pairs_occupancy(e) * PAIRS_WARPS;
-        const long long want = (6LL * warps + (long long)e->group_bound - 1) / std::max<long long>(1, e->group_bound);
-        p.gslices = (int)std::max<long long>(1, std::min<long long>(64, want));
-        e->gpart.ensure((size_t)p.gslices * e->max_atoms * PAIRS_NSUM);
+        // slices per group: about six work items per resident warp, so that the items taken
+        // last are short against the pass, at most one stencil row each (512 for boxes of a
+        // few groups: two-body pass of 16 and 96 atoms 0.36 and 0.49 ms with at most 64).
+        // The ATM lists keep at most 64: an apex's slices are prefixed one by one.
+        const long long warps = (long long)e->dev_sms * pairs_occupancy(e) * PAIRS_WARPS;
+        const long long groups = std::max<long long>(1, (long long)e->group_bound);
+        const long long want = (6 * warps + groups - 1) / groups;
+        int rows[2] = {1, 1};
+        for (const SG &q : e->sg) {
+            rows[0] = std::max(rows[0], q.st2b_n);
+            rows[1] = std::max(rows[1], q.stcb_n);
+        }
+        for (int k = 0; k < 2; ++k)
+            p.gslices_of[k] = (int)std::max<long long>(1, std::min<long long>(std::min(512, rows[k]), want));
+        p.gslices_of[2] = (int)std::max<long long>(1, std::min<long long>(64, want));
+        p.gslices = p.gslices_of[0];
+        // slices x atoms stays below this whatever the atom count of the next evaluation
+        const size_t most = std::min<size_t>(512 * (size_t)e->max_atoms, (size_t)(6 * warps) * 32 + 2 * (size_t)e->max_atoms);
+        e->gpart.ensure(most * PAIRS_NSUM);
         p.gpart = e->gpart.p;
     }
     p.pos_in = e->pos_in.p;
@@ -2184,11 +2199,13 @@ static unsigned long long engine_extra_visits(Engine *e) {
 }
 
 // ATM half lists of every apex (of the flagged ones in centre mode)
-static void launch_atm_lists(Engine *e, const KP &p, cudaStream_t s) {
+static void launch_atm_lists(Engine *e, const KP &p0, cudaStream_t s) {
+    KP p = p0;
     const int n = p.n, T = 256;
     const int gb = (n + T - 1) / T;
     const int gw = (int)(((long long)n * 32 + T - 1) / T);
     if (p.gslices > 0) {
+        p.gslices = p.gslices_of[2];
         const size_t sm = PAIRS_WARPS * 32 * (sizeof(double4) + sizeof(int));
         k_atm_list_g<false><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(p, e->gctl.p + 4);
         k_atm_list_prefix<<<gb, T, 0, s>>>(p);
@@ -2283,6 +2300,13 @@ static void atm_reference_pass(Engine *e) {
     e->opt = now;
 }
 
+static void launch_group_reduce(const KP &p, int what, cudaStream_t s) {
+    if (p.gslices >= 16)
+        k_group_reduce<true><<<(int)(((long long)p.n * 32 + 255) / 256), 256, 0, s>>>(p, what);
+    else
+        k_group_reduce<false><<<(p.n + 255) / 256, 256, 0, s>>>(p, what);
+}
+
 // stage 0: the whole evaluation; stage 1: everything up to the summed dE/dCN (written to
 // G_ext when given); stage 2: chain rule (dE/dCN read from G_ext), forces and reductions.
 // Stages 1 and 2 with an all-reduce of dE/dCN between them make a sharded evaluation.
@@ -2295,6 +2319,8 @@ static void launch_all(Engine *e, const KP &p0, cudaStream_t s, int stage = 0, d
     const int gw = (int)(((long long)n * 32 + T - 1) / T);
     cudaEvent_t *ev = e->ev;
     double *Gsum = G_ext ? G_ext : e->G.p;
+    KP pcn = p; // CN and chain-rule passes: their own slices
+    pcn.gslices = p.gslices_of[1];
     if (stage != 2) {
         e->eval_rank = p.shard_rank;
         e->eval_world = p.shard_world;
@@ -2319,10 +2345,10 @@ static void launch_all(Engine *e, const KP &p0, cudaStream_t s, int stage = 0, d
         if (p.gslices > 0) {
             const size_t sm = 64 + PAIRS_WARPS * 32 * (p.precision ? sizeof(float4) : sizeof(double4));
             if (p.precision)
-                k_cn_g<false><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(p, e->gctl.p + 1);
+                k_cn_g<false><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(pcn, e->gctl.p + 1);
             else
-                k_cn_g<true><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(p, e->gctl.p + 1);
-            k_group_reduce<<<gb, T, 0, s>>>(p, 1);
+                k_cn_g<true><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(pcn, e->gctl.p + 1);
+            launch_group_reduce(pcn, 1, s);
         } else if (p.precision)
             k_cn32<<<gw, T, 0, s>>>(p);
         else
@@ -2342,7 +2368,7 @@ static void launch_all(Engine *e, const KP &p0, cudaStream_t s, int stage = 0, d
                 k_twobody_g<NR, false><<<grid, PAIRS_WARPS * 32, pairs_smem(e), s>>>(p, e->gctl.p + 2);
             else
                 k_twobody_g<NR, true><<<grid, PAIRS_WARPS * 32, pairs_smem(e), s>>>(p, e->gctl.p + 2);
-            k_group_reduce<<<gb, T, 0, s>>>(p, 0);
+            launch_group_reduce(p, 0, s);
         } else if (p.precision)
             k_twobody32<NR><<<gw, T, (size_t)p.ne * p.ne * sizeof(float4), s>>>(p);
         else
@@ -2404,10 +2430,10 @@ static void launch_all(Engine *e, const KP &p0, cudaStream_t s, int stage = 0, d
     if (p.gslices > 0) {
         const size_t sm = 64 + PAIRS_WARPS * 32 * ((p.precision ? sizeof(float4) : sizeof(double4)) + sizeof(double));
         if (p.precision)
-            k_chain_g<false><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(p, Gsum, e->gctl.p + 3);
+            k_chain_g<false><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(pcn, Gsum, e->gctl.p + 3);
         else
-            k_chain_g<true><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(p, Gsum, e->gctl.p + 3);
-        k_group_reduce<<<gb, T, 0, s>>>(p, 2);
+            k_chain_g<true><<<e->dev_sms * 2, PAIRS_WARPS * 32, sm, s>>>(pcn, Gsum, e->gctl.p + 3);
+        launch_group_reduce(pcn, 2, s);
     } else if (p.precision)
         k_chain32<<<gw, T, 0, s>>>(p, Gsum);
     else

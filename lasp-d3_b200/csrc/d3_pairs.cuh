@@ -100,60 +100,43 @@ struct PairReal<true> {
     using R4 = double4;
 };
 
-// One (i, j) pair of the two-body term: energy (half), dE/dCN_i, force scalar fs with
-// F_i += fs r_ij and virial += fs r_ij (x) r_ij. y: partner's C6 row at the type of i.
-template <int NR, typename R>
-__device__ __forceinline__ void pair_term(const KP &p, R r2, const R *y, const R *wi, const R *dwi, R A6_or_R0,
-                                          R A8, R rr, R &e_half, R &G, R &fs) {
-    R c6 = 0, dc6 = 0;
-#pragma unroll
-    for (int b = 0; b < NR; ++b) {
-        c6 = fma(y[b], wi[b], c6);
-        dc6 = fma(y[b], dwi[b], dc6);
-    }
-    const R c8 = c6 * rr, dc8 = dc6 * rr;
-    const R s6 = (R)p.s6, s8 = (R)p.s8;
-    R E6, E8;
+// One (i, j) pair of the two-body term per unit of C6: energy C6 S, dE/dCN_i = dC6 S, force
+// scalar -6 C6 T with F_i += -6 C6 T r_ij and virial += -6 C6 T r_ij (x) r_ij (the caller
+// applies the constants, and 1/2 to the energy). q8 = s8 3 r2r4_i r2r4_j. The FP64 form uses
+// reciprocals and roots refined by one third-order step instead of divisions: 11 FP64
+// operations for S and T (Becke-Johnson) where four IEEE divisions took over 60.
+template <typename R>
+__device__ __forceinline__ R pair_rcp(R x) {
+    if constexpr (sizeof(R) == 4)
+        return sfu_rcp(x);
+    else
+        return rcp_nr(x);
+}
+template <typename R>
+__device__ __forceinline__ void pair_term(const KP &p, R r2, R A6_or_R0, R A8, R q8, R &S, R &T) {
+    const R s6 = (R)p.s6;
     if (p.damping == 1) {
-        const R r4 = r2 * r2, r6 = r4 * r2, r8 = r4 * r4;
-        R i6, i8;
-        if constexpr (sizeof(R) == 4) {
-            i6 = sfu_rcp(r6 + A6_or_R0);
-            i8 = sfu_rcp(r8 + A8);
-        } else {
-            i6 = 1.0 / (r6 + A6_or_R0);
-            i8 = 1.0 / (r8 + A8);
-        }
-        E6 = s6 * c6 * i6;
-        E8 = s8 * c8 * i8;
-        G = s6 * dc6 * i6 + s8 * dc8 * i8;
-        fs = (R)-6 * E6 * r4 * i6 - (R)8 * E8 * r6 * i8;
+        const R r4 = r2 * r2;
+        const R i6 = pair_rcp<R>(fma(r4, r2, A6_or_R0)), i8 = pair_rcp<R>(fma(r4, r4, A8));
+        const R x6 = s6 * i6, x8 = q8 * i8;
+        S = x6 + x8;
+        T = r4 * fma((R)(4.0 / 3.0) * x8 * i8, r2, x6 * i6);
     } else {
         R ir;
         if constexpr (sizeof(R) == 4)
             ir = sfu_rsqrt(r2);
         else
-            ir = 1.0 / sqrt(r2);
-        const R ir2 = ir * ir, ir6 = ir2 * ir2 * ir2, ir8 = ir6 * ir2;
-        const R R0 = A6_or_R0;
-        const R x6 = (R)p.p1 * R0 * ir, x8 = (R)p.p2 * R0 * ir;
-        const R x6_2 = x6 * x6, x6_4 = x6_2 * x6_2, x6_8 = x6_4 * x6_4, x6_14 = x6_8 * x6_4 * x6_2;
-        const R x8_2 = x8 * x8, x8_4 = x8_2 * x8_2, x8_8 = x8_4 * x8_4, x8_16 = x8_8 * x8_8;
-        R f6, f8;
-        if constexpr (sizeof(R) == 4) {
-            f6 = sfu_rcp(fmaf(6.0f, x6_14, 1.0f));
-            f8 = sfu_rcp(fmaf(6.0f, x8_16, 1.0f));
-        } else {
-            f6 = 1.0 / (1.0 + 6.0 * x6_14);
-            f8 = 1.0 / (1.0 + 6.0 * x8_16);
-        }
-        const R df6 = (R)84 * f6 * f6 * x6_14 * ir, df8 = (R)96 * f8 * f8 * x8_16 * ir;
-        E6 = s6 * c6 * f6 * ir6;
-        E8 = s8 * c8 * f8 * ir8;
-        G = s6 * f6 * dc6 * ir6 + s8 * f8 * dc8 * ir8;
-        fs = s6 * c6 * ((R)-6 * f6 * ir8 + df6 * ir6 * ir) + s8 * c8 * ((R)-8 * f8 * ir8 * ir2 + df8 * ir8 * ir);
+            ir = rsqrt_nr(r2);
+        const R ir2 = ir * ir, ir4 = ir2 * ir2, ir6 = ir4 * ir2, ir8 = ir4 * ir4;
+        const R x6 = (R)p.p1 * A6_or_R0 * ir, x8 = (R)p.p2 * A6_or_R0 * ir;
+        const R x6_2 = x6 * x6, x6_4 = x6_2 * x6_2, x6_14 = x6_4 * x6_4 * x6_4 * x6_2;
+        const R x8_2 = x8 * x8, x8_4 = x8_2 * x8_2, x8_8 = x8_4 * x8_4;
+        const R f6 = pair_rcp<R>(fma((R)6 * x6_14, (R)1, (R)1)), f8 = pair_rcp<R>(fma((R)6 * x8_8, x8_8, (R)1));
+        // f6' = 14 x6^14 f6 = 7/3 (1 - f6), f8' = 12 x8^16 f8 = 2 (1 - f8)
+        const R y6 = s6 * f6 * ir6, y8 = q8 * f8 * ir8;
+        S = y6 + y8;
+        T = ir2 * (y6 * fma((R)(-7.0 / 3.0), (R)1 - f6, (R)1) + (R)(4.0 / 3.0) * y8 * fma((R)-2, (R)1 - f8, (R)1));
     }
-    e_half = (R)0.5 * (E6 + E8);
 }
 
 // shared memory of one warp: 32 partner positions, their C6 rows at every type (two-body)
@@ -251,19 +234,19 @@ __device__ __forceinline__ R cn_pair(const KP &p, R r2, R rsum, R *dcn_over_r) {
 }
 
 template <int NR, bool F64>
-__global__ void __launch_bounds__(PAIRS_WARPS * 32, F64 ? 1 : 2) k_twobody_g(KP p, int *work) {
+__global__ void __launch_bounds__(PAIRS_WARPS * 32, 2) k_twobody_g(KP p, int *work) {
     using R = typename PairReal<F64>::R;
     using R4 = typename PairReal<F64>::R4;
     extern __shared__ __align__(16) unsigned char smp[];
     const int ne = p.ne;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // per type pair: BJ A^6, A^8 (zero damping: R0) and 3 r2r4_i r2r4_j
+    // per type pair: BJ A^6, A^8 (zero damping: R0) and s8 3 r2r4_i r2r4_j
     R *ptab = reinterpret_cast<R *>(smp);
     for (int k = threadIdx.x; k < ne * ne; k += blockDim.x) {
         const double *pa = p.pairA + (size_t)k * 4;
         ptab[3 * k] = (R)pa[0];
         ptab[3 * k + 1] = (R)pa[1];
-        ptab[3 * k + 2] = (R)(3.0 * p.r2r4[k / ne] * p.r2r4[k % ne]);
+        ptab[3 * k + 2] = (R)(p.s8 * 3.0 * p.r2r4[k / ne] * p.r2r4[k % ne]);
     }
     __syncthreads();
     const size_t tab_bytes = ((size_t)3 * ne * ne * sizeof(R) + 15) & ~(size_t)15;
@@ -333,22 +316,32 @@ __global__ void __launch_bounds__(PAIRS_WARPS * 32, F64 ? 1 : 2) k_twobody_g(KP 
                 if (!(act0 || act1)) continue;
                 npair += (act0 ? 1 : 0) + (act1 ? 1 : 0);
                 const R *tp0 = ptab + 3 * (ti * ne + (int)x0.w), *tp1 = ptab + 3 * (ti * ne + (int)x1.w);
-                R eh0, Gt0, fs0, eh1, Gt1, fs1;
-                pair_term<NR, R>(p, act0 ? r20 : rc2, sY + jj * rowlen + ti * NR, wi, dwi, tp0[0], tp0[1], tp0[2], eh0,
-                                 Gt0, fs0);
-                pair_term<NR, R>(p, act1 ? r21 : rc2, sY + j1 * rowlen + ti * NR, wi, dwi, tp1[0], tp1[1], tp1[2], eh1,
-                                 Gt1, fs1);
-                if (!act0) eh0 = Gt0 = fs0 = (R)0;
-                if (!act1) eh1 = Gt1 = fs1 = (R)0;
-                e += eh0 + eh1;
-                Gd += (double)Gt0 + (double)Gt1;
-                fx = fma(fs0, dx0, fma(fs1, dx1, fx));
-                fy = fma(fs0, dy0, fma(fs1, dy1, fy));
-                fz = fma(fs0, dz0, fma(fs1, dz1, fz));
-                const R fdx0 = fs0 * dx0, fdy0 = fs0 * dy0, fdx1 = fs1 * dx1, fdy1 = fs1 * dy1;
+                R S0, T0, S1, T1;
+                pair_term<R>(p, act0 ? r20 : rc2, tp0[0], tp0[1], tp0[2], S0, T0);
+                pair_term<R>(p, act1 ? r21 : rc2, tp1[0], tp1[1], tp1[2], S1, T1);
+                // C6 = y . w_i and its CN derivative; y: the partner's C6 row at the type of i
+                const R *y0 = sY + jj * rowlen + ti * NR, *y1 = sY + j1 * rowlen + ti * NR;
+                R c60 = y0[0] * wi[0], dc0 = y0[0] * dwi[0], c61 = y1[0] * wi[0], dc1 = y1[0] * dwi[0];
+#pragma unroll
+                for (int b = 1; b < NR; ++b) {
+                    c60 = fma(y0[b], wi[b], c60);
+                    dc0 = fma(y0[b], dwi[b], dc0);
+                    c61 = fma(y1[b], wi[b], c61);
+                    dc1 = fma(y1[b], dwi[b], dc1);
+                }
+                if (!act0) c60 = dc0 = (R)0;
+                if (!act1) c61 = dc1 = (R)0;
+                e = fma(c60, S0, fma(c61, S1, e));
+                Gd += (double)(dc0 * S0) + (double)(dc1 * S1);
+                const R fs0 = c60 * T0, fs1 = c61 * T1;
+                const R fdx0 = fs0 * dx0, fdy0 = fs0 * dy0, fdz0 = fs0 * dz0;
+                const R fdx1 = fs1 * dx1, fdy1 = fs1 * dy1, fdz1 = fs1 * dz1;
+                fx += fdx0 + fdx1;
+                fy += fdy0 + fdy1;
+                fz += fdz0 + fdz1;
                 vxx = fma(fdx0, dx0, fma(fdx1, dx1, vxx));
                 vyy = fma(fdy0, dy0, fma(fdy1, dy1, vyy));
-                vzz = fma(fs0 * dz0, dz0, fma(fs1 * dz1, dz1, vzz));
+                vzz = fma(fdz0, dz0, fma(fdz1, dz1, vzz));
                 vxy = fma(fdx0, dy0, fma(fdx1, dy1, vxy));
                 vxz = fma(fdx0, dz0, fma(fdx1, dz1, vxz));
                 vyz = fma(fdy0, dz0, fma(fdy1, dz1, vyz));
@@ -367,13 +360,13 @@ __global__ void __launch_bounds__(PAIRS_WARPS * 32, F64 ? 1 : 2) k_twobody_g(KP 
         });
         if (iv) {
             double *o = p.gpart + ((size_t)it.sl * p.n + i) * PAIRS_NSUM;
-            o[0] = E;
+            o[0] = 0.5 * E;
             o[1] = Gd;
-            o[2] = FX;
-            o[3] = FY;
-            o[4] = FZ;
+            o[2] = -6.0 * FX;
+            o[3] = -6.0 * FY;
+            o[4] = -6.0 * FZ;
 #pragma unroll
-            for (int k = 0; k < 6; ++k) o[5 + k] = V[k];
+            for (int k = 0; k < 6; ++k) o[5 + k] = -6.0 * V[k];
         }
     }
     for (int o = 16; o > 0; o >>= 1) npair += __shfl_xor_sync(0xffffffffu, npair, o);
@@ -520,19 +513,28 @@ __global__ void __launch_bounds__(PAIRS_WARPS * 32, 2) k_chain_g(KP p, const dou
 }
 
 // per atom: the slices' sums in a fixed order. what: 0 two-body (energy, dE/dCN, force,
-// virial), 1 CN, 2 chain rule (force, virial)
+// virial), 1 CN, 2 chain rule (force, virial). WIDE: one warp per atom (many slices of few
+// atoms; one thread adds 512 slices in 0.3 ms), else one thread
+template <bool WIDE>
 __global__ void k_group_reduce(KP p, int what) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = WIDE ? t >> 5 : t;
     if (i >= p.n) return;
     const int nsum = what == 0 ? PAIRS_NSUM : (what == 1 ? 1 : 9);
     double acc[PAIRS_NSUM];
 #pragma unroll
     for (int k = 0; k < PAIRS_NSUM; ++k) acc[k] = 0.0;
-    for (int s = 0; s < p.gslices; ++s) {
+    for (int s = WIDE ? (t & 31) : 0; s < p.gslices; s += WIDE ? 32 : 1) {
         const double *o = p.gpart + ((size_t)s * p.n + i) * PAIRS_NSUM;
 #pragma unroll
         for (int k = 0; k < PAIRS_NSUM; ++k)
             if (k < nsum) acc[k] += o[k];
+    }
+    if (WIDE) {
+#pragma unroll
+        for (int k = 0; k < PAIRS_NSUM; ++k)
+            if (k < nsum) acc[k] = warp_sum(acc[k]);
+        if ((t & 31) != 0) return;
     }
     const double sc = -1.0 / (2.0 * p.sg[p.sid[i]].vol);
     if (what == 1) {
