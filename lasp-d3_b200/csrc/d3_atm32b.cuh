@@ -40,7 +40,10 @@
 // with the x rows staged per type -> 49 % with the y rows; long-scoreboard stalls of the
 // synchronous y gather removed by the cp.async double buffer; warp instructions -22 % with
 // the packed pairs, which leaves the kernel bound by the latency of the packed chains
-// (2 warps of 243 registers per scheduler, four independent chains).
+// (2 warps of 243 registers per scheduler, four independent chains). Regrouped triplet term
+// (94 -> 80 packed instructions for two visits): ATM pass of the 20,000-atom box 186.3 ->
+// 180.7 ms; now bound by the shared-memory pipe (64 % of its wavefronts) and the FMA pipe
+// (57 %) together: 13 or 14 warps per CTA bring nothing.
 
 // longest list this kernel takes (longer lists: k_atm32): chosen per launch, a multiple of
 // 512 in [ATMB_MCAP_MIN, ATMB_MCAP_MAX], as large as the shared memory left by the warps allows
@@ -203,12 +206,12 @@ __device__ __forceinline__ float atmb_dot2(const float *r, const AtmbVec<NR> &v)
     return fmaf(r[NR - 1], v.l, acc.x) + acc.y;
 }
 
-// per-row constants of the x entry as (v, v) pairs for the packed arithmetic of two visits;
-// gq carries the factor (4/3)^16, c1 = -0.75 d1, d1x3 = 3 d1; w, dw its own C6 weights and
-// their CN derivatives
+// per-row constants of the x entry as (v, v) pairs for the packed arithmetic of two visits:
+// position, d, 1/d, h = -3/4 / d, p = sqrt(C6) / r^3, g = 6 (4/3)^16 (r0^2/d)^(8/3); w, dw its
+// own C6 weights and their CN derivatives
 template <int NR>
 struct AtmbX2 {
-    float2 vx, vy, vz, d1, ir1, id1, sq, gq, c1, d1x3;
+    float2 vx, vy, vz, d1, id1, h, p, g;
     AtmbVec<NR> w, dw;
     int jx;
     bool qa;
@@ -281,23 +284,26 @@ struct AtmbXSums2 {
 // Two (possible) visits of entry x, with the staged partners k0 and k1 = k0 + 1 (mod 32)
 // of two consecutive steps, in packed f32x2 arithmetic (component x: k0, y: k1): triplet
 // terms, x-side sums into xt, y-side sums into ys, virial corrections where the energy and
-// force weights differ. P0 = (x, x', y, y'), P1 = (z, z', d2, d2') of the two partners.
+// force weights differ. P0 = (x, x', y, y'), P1 = (z, z', d2, d2') of the two partners,
+// yQ0 = (1/d, 1/d', p, p'), yQ1 = (g, g').
 // Branch-free: an out-of-range pair (act false) runs on finite stand-in values (lanes
 // without entry and padding partners sit at far, distinct points with positive C6 rows)
-// with zero weights. With P = t1 t2 t3 (t1 = d1 + d2 - d3 ...), the angular term is
-// A = (1 + 3/8 P / (d1 d2 d3)) / (r1 r2 r3)^3 and its side derivatives
-// dA/dr_k / r_k = q52 G_k, G_k = 15/8 P + 3 d1 d2 d3 - 3/4 d_k (T - 2 t_ij),
-// T = t12 + t13 + t23 (t_ij the product of the two t's without t_k). Signs are carried in
-// the constants (f32x2 has add, mul and fma only): nw = -w, Em = -E, ndfd = -dfd.
+// with zero weights. The terms are those of k_atm64 (d3_atm.cuh):
+//     C = p1 p2 p3, h = -3/4 / (d1 d2 d3), u = t1 t2 t3 h, B = 1 - u/2, -E = C fd B,
+//     f_k = S / d_k + C fd h n_k, S = C fd (3 - 5/2 u - 16/3 (1 - fd) B)
+// with n_k the derivatives of t1 t2 t3: 80 packed instructions for two visits, 94 when each
+// side's derivative was formed from its own polynomial. Signs are carried in the constants
+// (f32x2 has add, mul and fma only).
 template <int NR, bool SIMPLE>
 __device__ __forceinline__ void atmb_visit2(const AtmbX2<NR> &X, int k0, float2 d3in, bool act0, bool act1,
-                                            const float4 P0, const float4 P1, const float4 *yQ0, const float4 *yQ1,
+                                            const float4 P0, const float4 P1, const float4 *yQ0, const float2 *yQ1,
                                             const float4 *yrow, int a, bool ref, bool force_scaled,
                                             AtmbXSums2<SIMPLE> &xt, AtmbYSums2<SIMPLE> &ys) {
     const int k1 = (k0 + 1) & 31;
-    const float2 ONE = make_float2(1.0f, 1.0f), M1 = make_float2(-1.0f, -1.0f), M2 = make_float2(-2.0f, -2.0f);
+    const float2 ONE = make_float2(1.0f, 1.0f), M1 = make_float2(-1.0f, -1.0f);
     const float2 d3 = make_float2(act0 ? d3in.x : X.d1.x, act1 ? d3in.y : X.d1.x);
-    const float4 Q0 = yQ0[k0], Q1 = yQ1[k0]; // (ir, ir', id2, id2'), (s, s', g, g')
+    const float4 Q0 = yQ0[k0]; // (id2, id2', p, p')
+    const float2 g2 = yQ1[k0], id2 = make_float2(Q0.x, Q0.y);
     AtmbRow<NR> R0, R1; // the partners' rows at the x entry's type
     R0.load(yrow, k0);
     R1.load(yrow, k1);
@@ -308,9 +314,7 @@ __device__ __forceinline__ void atmb_visit2(const AtmbX2<NR> &X, int k0, float2 
     const float2 dcx = make_float2(atmb_dot2<NR>(R0.Y, X.dw), atmb_dot2<NR>(R1.Y, X.dw)); // dC6_xy/dCN_x
     const float2 dcy = make_float2(atmb_dot2<NR>(R0.D, X.w), atmb_dot2<NR>(R1.D, X.w));   // dC6_xy/dCN_y
     const float2 is3 = make_float2(sfu_rsqrt(c6.x), sfu_rsqrt(c6.y));
-    const float2 s3 = __fmul2_rn(c6, is3);
-    const float2 is3q = __fmul2_rn(is3, is3);
-    const float2 lam_xy = __fmul2_rn(dcx, is3q), lam_yx = __fmul2_rn(dcy, is3q);
+    const float2 p3 = __fmul2_rn(__fmul2_rn(__fmul2_rn(c6, is3), ir3), id3); // sqrt(C6) / r^3
     // (r0_xy^2 / d3)^(8/3)
     const float2 lgu = __fmul2_rn(make_float2(sfu_log2(R0.r0sq * id3.x), sfu_log2(R1.r0sq * id3.y)),
                                   make_float2(8.0f / 3.0f, 8.0f / 3.0f));
@@ -329,37 +333,32 @@ __device__ __forceinline__ void atmb_visit2(const AtmbX2<NR> &X, int k0, float2 
         wf = make_float2(act0 ? wf0 : 0.0f, act1 ? wf1 : 0.0f);
     }
     const float2 d1 = X.d1, d2 = make_float2(P1.z, P1.w);
-    const float2 irsq = __fmul2_rn(__fmul2_rn(X.id1, make_float2(Q0.z, Q0.w)), id3);
-    const float2 ir9 = __fmul2_rn(__fmul2_rn(__fmul2_rn(irsq, X.ir1), make_float2(Q0.x, Q0.y)), ir3);
+    const float2 C = __fmul2_rn(__fmul2_rn(X.p, make_float2(Q0.z, Q0.w)), p3);
+    const float2 h = __fmul2_rn(__fmul2_rn(X.h, id2), id3);
+    const float2 m12 = __ffma2_rn(d2, M1, d1);                // d1 - d2
     const float2 t1 = __ffma2_rn(d3, M1, __fadd2_rn(d1, d2)); // d1 + d2 - d3
-    const float2 t2 = __fadd2_rn(__ffma2_rn(d2, M1, d1), d3); // d1 - d2 + d3
-    const float2 t3 = __fadd2_rn(__ffma2_rn(d1, M1, d2), d3); // -d1 + d2 + d3
+    const float2 t2 = __fadd2_rn(m12, d3);                    // d1 - d2 + d3
+    const float2 t3 = __ffma2_rn(m12, M1, d3);                // -d1 + d2 + d3
     const float2 t12 = __fmul2_rn(t1, t2), t13 = __fmul2_rn(t1, t3), t23 = __fmul2_rn(t2, t3);
-    const float2 P = __fmul2_rn(t12, t3);
-    const float2 T = __fadd2_rn(__fadd2_rn(t12, t13), t23);
-    const float2 Aang = __fmul2_rn(__ffma2_rn(__fmul2_rn(make_float2(0.375f, 0.375f), P), irsq, ONE), ir9);
-    const float2 q52 = __fmul2_rn(ir9, irsq);
-    const float2 base = __ffma2_rn(make_float2(1.875f, 1.875f), P, __fmul2_rn(__fmul2_rn(X.d1x3, d2), d3));
-    const float2 G1 = __ffma2_rn(X.c1, __ffma2_rn(M2, t12, T), base);
-    const float2 G2 = __ffma2_rn(__fmul2_rn(make_float2(-0.75f, -0.75f), d2), __ffma2_rn(M2, t13, T), base);
-    const float2 G3 = __ffma2_rn(__fmul2_rn(make_float2(-0.75f, -0.75f), d3), __ffma2_rn(M2, t23, T), base);
-    const float2 x16 = __fmul2_rn(__fmul2_rn(X.gq, make_float2(Q1.z, Q1.w)), g3);
-    const float2 den = __ffma2_rn(make_float2(6.0f, 6.0f), x16, ONE);
+    const float2 u = __fmul2_rn(__fmul2_rn(t12, t3), h);
+    const float2 B = __ffma2_rn(make_float2(-0.5f, -0.5f), u, ONE);
+    const float2 den = __ffma2_rn(__fmul2_rn(X.g, g2), g3, ONE);
     const float2 fd = make_float2(sfu_rcp(den.x), sfu_rcp(den.y));
-    const float2 ndfd = __fmul2_rn(__fmul2_rn(__fmul2_rn(make_float2(-32.0f, -32.0f), x16), fd), fd);
-    const float2 nC9 = __fmul2_rn(__fmul2_rn(X.sq, make_float2(Q1.x, Q1.y)), s3); // -C9
-    const float2 nC9fd = __fmul2_rn(nC9, fd);
-    const float2 Em = __fmul2_rn(nC9fd, Aang); // -E
-    const float2 Ap = __fmul2_rn(nC9fd, q52), nBp = __fmul2_rn(__fmul2_rn(nC9, Aang), ndfd);
-    const float2 f1 = __fmul2_rn(__ffma2_rn(Ap, G1, nBp), X.id1);
-    const float2 f2 = __fmul2_rn(__ffma2_rn(Ap, G2, nBp), make_float2(Q0.z, Q0.w));
-    const float2 f3 = __fmul2_rn(__ffma2_rn(Ap, G3, nBp), id3);
-    const float2 wE = __fmul2_rn(nw, Em);
+    const float2 k16 = __ffma2_rn(make_float2(16.0f / 3.0f, 16.0f / 3.0f), fd, make_float2(-16.0f / 3.0f, -16.0f / 3.0f));
+    const float2 Ef = __fmul2_rn(C, fd);
+    const float2 S = __fmul2_rn(Ef, __ffma2_rn(k16, B, __ffma2_rn(make_float2(-2.5f, -2.5f), u, make_float2(3.0f, 3.0f))));
+    const float2 Eh = __fmul2_rn(Ef, h);
+    const float2 dt = __ffma2_rn(t12, M1, t23); // t23 - t12
+    const float2 f1 = __ffma2_rn(Eh, __fadd2_rn(t13, dt), __fmul2_rn(X.id1, S));
+    const float2 f2 = __ffma2_rn(Eh, __ffma2_rn(t13, M1, __fadd2_rn(t12, t23)), __fmul2_rn(id2, S));
+    const float2 f3 = __ffma2_rn(Eh, __ffma2_rn(dt, M1, t13), __fmul2_rn(id3, S));
+    const float2 wE = __fmul2_rn(nw, __fmul2_rn(Ef, B));
+    const float2 q = __fmul2_rn(wE, __fmul2_rn(is3, is3)); // w E / C6_xy
     const float2 wf3 = __fmul2_rn(wf, f3);
     const float2 f13 = __fadd2_rn(f1, f3), f23 = __fadd2_rn(f2, f3);
     const float2 yx = make_float2(P0.x, P0.y), yy = make_float2(P0.z, P0.w), yz = make_float2(P1.x, P1.y);
     xt.SE = __fadd2_rn(xt.SE, wE);
-    xt.SD = __ffma2_rn(wE, lam_xy, xt.SD);
+    xt.SD = __ffma2_rn(q, dcx, xt.SD);
     xt.SF = __ffma2_rn(wf, f13, xt.SF);
     xt.Wx = __ffma2_rn(wf3, yx, xt.Wx);
     xt.Wy = __ffma2_rn(wf3, yy, xt.Wy);
@@ -367,7 +366,7 @@ __device__ __forceinline__ void atmb_visit2(const AtmbX2<NR> &X, int k0, float2 
     // minus the y entry's force: wf f3 v_x - wf (f2 + f3) v_y (SIMPLE: -wf = nw)
     const float2 nwf23 = __fmul2_rn(SIMPLE ? nw : __fmul2_rn(wf, M1), f23);
     ys.SE = __fadd2_rn(ys.SE, wE);
-    ys.SD = __ffma2_rn(wE, lam_yx, ys.SD);
+    ys.SD = __ffma2_rn(q, dcy, ys.SD);
     ys.NFx = __ffma2_rn(wf3, X.vx, __ffma2_rn(nwf23, yx, ys.NFx));
     ys.NFy = __ffma2_rn(wf3, X.vy, __ffma2_rn(nwf23, yy, ys.NFy));
     ys.NFz = __ffma2_rn(wf3, X.vz, __ffma2_rn(nwf23, yz, ys.NFz));
@@ -424,7 +423,7 @@ __global__ void __launch_bounds__((NBUF == 2 ? ATMB_MAXW : ATMB_MAXW1) * 32, 1) 
     if (p.atm_off[p.n] > p.atm_cap) return; // list overflowed: the host grows it and re-runs
     for (int k = tid; k < ne * ne; k += blockDim.x) r0sq[k] = (float)(p.r0ab[k] * p.r0ab[k]);
     static_assert(NR == 5 || NR == 7, "reference counts of the parameter tables");
-    const float x16c = (float)(4294967296.0 / 43046721.0); // (4/3)^16
+    const float x16c = (float)(6.0 * 4294967296.0 / 43046721.0); // 6 (4/3)^16
     const float ratm2f = (float)p.ratm2;
     const bool force_scaled = p.atm_force_scaled != 0;
     const double rc = sqrt(p.ratm2);
@@ -536,8 +535,8 @@ __global__ void __launch_bounds__((NBUF == 2 ? ATMB_MAXW : ATMB_MAXW1) * 32, 1) 
                 dca += yq[b] * dwa[b];
             }
             sA[pos] = make_float4((float)vx, (float)vy, (float)vz, (float)d2);
-            sB[pos] = make_float4((float)(1.0 / sqrt(d2)), (float)(1.0 / d2), (float)sqrt(c6),
-                                  (float)pow((double)r0sq[ta * ne + tp] / d2, 8.0 / 3.0));
+            const double id = 1.0 / d2;
+            sB[pos] = make_float4((float)id, (float)(sqrt(c6 * id) * id), (float)pow((double)r0sq[ta * ne + tp] * id, 8.0 / 3.0), 0.f);
             sJ[pos] = make_float4(__int_as_float(jp), __int_as_float(tp), (float)(dcq / c6), (float)(dca / c6));
             sjy[pos] = jp; // this thread's own slot: the entry number it replaces was read above
         }
@@ -569,10 +568,11 @@ __global__ void __launch_bounds__((NBUF == 2 ? ATMB_MAXW : ATMB_MAXW1) * 32, 1) 
         // sums of this lane's x entry
         const AtmbCarry apx{reinterpret_cast<double *>(wbase + NBUF * bufq * sizeof(float4)) + lane};
         const AtmbCarry xs{apx.p + 6 * 32}; // SE SD SF Wx Wy Wz, weighted form also Ux Uy Uz
-        // positions (x, x', y, y'), (z, z', d2, d2') and constants (ir, ir', id2, id2'),
-        // (s, s', g, g') of the current y block, entries k and k + 1 at slot k
+        // positions (x, x', y, y'), (z, z', d2, d2') and constants (1/d, 1/d', p, p'),
+        // (g, g') of the current y block, entries k and k + 1 at slot k
         float4 *yP0 = reinterpret_cast<float4 *>(wbase + NBUF * bufq * sizeof(float4) + ATMB_NCARRY * 32 * sizeof(double));
-        float4 *yP1 = yP0 + 32, *yQ0 = yP1 + 32, *yQ1 = yQ0 + 32;
+        float4 *yP1 = yP0 + 32, *yQ0 = yP1 + 32;
+        float2 *yQ1 = reinterpret_cast<float2 *>(yQ0 + 32);
 #pragma unroll
         for (int q = 0; q < 6; ++q) apx[q] = 0.0;
         // rows are handed out in order (row A holds nb - A block pairs, so the dearest go
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__((NBUF == 2 ? ATMB_MAXW : ATMB_MAXW1) * 32, 1) 
             const bool xvalid = xe < m;
             // a lane without entry sits at a far point (distinct from the padding partners)
             // with weights (1, 0, ...), so its visits stay finite
-            float vx = 3e4f, vy = 3e4f, vz = 3e4f, d1 = 1.f, ir1 = 1.f, id1 = 1.f, sq = 0.f, gq = 0.f;
+            float vx = 3e4f, vy = 3e4f, vz = 3e4f, d1 = 1.f, id1 = 1.f, px = 0.f, gx = 0.f;
             int jx = -1, tx = 0;
             float wx[NR], dwx[NR];
 #pragma unroll
@@ -600,10 +600,9 @@ __global__ void __launch_bounds__((NBUF == 2 ? ATMB_MAXW : ATMB_MAXW1) * 32, 1) 
                 vy = qa4.y;
                 vz = qa4.z;
                 d1 = qa4.w;
-                ir1 = qb4.x;
-                id1 = qb4.y;
-                sq = qb4.z;
-                gq = qb4.w * x16c;
+                id1 = qb4.x;
+                px = qb4.y;
+                gx = qb4.z * x16c;
                 jx = __float_as_int(qj4.x);
                 tx = __float_as_int(qj4.y);
 #pragma unroll
@@ -618,12 +617,10 @@ __global__ void __launch_bounds__((NBUF == 2 ? ATMB_MAXW : ATMB_MAXW1) * 32, 1) 
             X.vy = make_float2(vy, vy);
             X.vz = make_float2(vz, vz);
             X.d1 = make_float2(d1, d1);
-            X.ir1 = make_float2(ir1, ir1);
             X.id1 = make_float2(id1, id1);
-            X.sq = make_float2(sq, sq);
-            X.gq = make_float2(gq, gq);
-            X.c1 = make_float2(-0.75f * d1, -0.75f * d1);
-            X.d1x3 = make_float2(3.0f * d1, 3.0f * d1);
+            X.h = make_float2(-0.75f * id1, -0.75f * id1);
+            X.p = make_float2(px, px);
+            X.g = make_float2(gx, gx);
 #pragma unroll
             for (int i = 0; i < (NR - 1) / 2; ++i) {
                 X.w.p[i] = make_float2(wx[2 * i], wx[2 * i + 1]);
@@ -663,7 +660,7 @@ __global__ void __launch_bounds__((NBUF == 2 ? ATMB_MAXW : ATMB_MAXW1) * 32, 1) 
                     // padding partner: a far point with zero C6 share that fails every
                     // distance test; unit rows keep C6_xy positive
                     ya[lane] = make_float4(-3e4f, -3e4f, -3e4f, 1.f);
-                    yb[lane] = make_float4(1.f, 1.f, 0.f, 0.f);
+                    yb[lane] = make_float4(1.f, 0.f, 0.f, 0.f);
                     for (int t = 0; t < ne; ++t) AtmbRowFill<NR>::padding(rows + t * RQ * 32 + lane);
                 }
             };
@@ -697,11 +694,11 @@ __global__ void __launch_bounds__((NBUF == 2 ? ATMB_MAXW : ATMB_MAXW1) * 32, 1) 
                     const float a1x = __shfl_sync(0xffffffffu, a0.x, nx), a1y = __shfl_sync(0xffffffffu, a0.y, nx);
                     const float a1z = __shfl_sync(0xffffffffu, a0.z, nx), a1w = __shfl_sync(0xffffffffu, a0.w, nx);
                     const float b1x = __shfl_sync(0xffffffffu, b0.x, nx), b1y = __shfl_sync(0xffffffffu, b0.y, nx);
-                    const float b1z = __shfl_sync(0xffffffffu, b0.z, nx), b1w = __shfl_sync(0xffffffffu, b0.w, nx);
+                    const float b1z = __shfl_sync(0xffffffffu, b0.z, nx);
                     yP0[lane] = make_float4(a0.x, a1x, a0.y, a1y);
                     yP1[lane] = make_float4(a0.z, a1z, a0.w, a1w);
                     yQ0[lane] = make_float4(b0.x, b1x, b0.y, b1y);
-                    yQ1[lane] = make_float4(b0.z, b1z, b0.w, b1w);
+                    yQ1[lane] = make_float2(b0.z, b1z);
                 }
                 __syncwarp();
                 AtmbXSums2<simple> xt{};    // x side of this block pair (two partial sums)
