@@ -116,8 +116,9 @@ enum {
     D3_OPT_BIN_DIVISOR = 4,      /* cell-list bin width = smallest cutoff / value (1..32, default 6) */
     D3_OPT_ATM_TILE = 5,         /* ATM partner tile entries (0 = automatic) */
     D3_OPT_ATM_CTAS_PER_SM = 6,  /* persistent ATM CTAs per SM (0 = occupancy limit) */
-    D3_OPT_ATM_SCHEDULE = 8,     /* precision-form ATM: 0 (default) block pairs, each triplet
-                                    visited once; 1 mirror-symmetric, each triplet twice */
+    D3_OPT_ATM_SCHEDULE = 8,     /* ATM: 0 (default) block pairs, each triplet visited once
+                                    (FP64: where apexes and lists are large enough for it);
+                                    1 mirror-symmetric, each triplet twice */
     D3_OPT_ATM_LIST_CAPACITY = 9, /* ATM half-list capacity in entries (0 = estimated from the
                                     density, the default). A synchronous evaluation whose
                                     list overflows grows it and runs again; an asynchronous

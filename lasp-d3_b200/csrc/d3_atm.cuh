@@ -43,7 +43,9 @@
 // ATM pass on a B200, one thread per entry with a private partner mask -> this kernel:
 // 16-atom metal cell 26.8 -> 0.38 ms, 96-atom water box 36.2 -> 2.65 ms (their few apexes
 // are split over all CTAs), 777 atoms 49.4 -> 20.7 ms, 2,000 atoms 73.3 -> 50.0 ms,
-// 20,000-atom box 745 -> 441 ms.
+// 20,000-atom box 745 -> 441 ms. Large systems take k_atm64b (d3_atm64b.cuh), which visits a
+// triplet once; this kernel keeps few apexes, short lists, lists beyond k_atm64b's capacity,
+// many types and the surrogate fallback.
 
 constexpr int ATM64_THREADS = 512;  // threads of all CTAs of an SM together
 constexpr int ATM64_ROWS = 4096;    // entries set up at once (longer lists: in parts)
@@ -149,6 +151,33 @@ __device__ __forceinline__ Atm64Row atm64_entry(const KP &p, const SG &g, const 
 // keeps once per warp: loops bounded by it need no divergence checks at every vote and
 // shuffle inside
 __device__ __forceinline__ int warp_uniform(int v) { return (int)__reduce_max_sync(0xffffffffu, v); }
+
+// exclusive scan of the cell counts by the whole CTA: a run of 32 cells per warp and step
+__device__ __forceinline__ void atm64_scan(int *cells, int ncell, int *s_tot) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int run = (ncell / 32 + nw - 1) / nw; // steps per warp
+    int carry = 0;
+    for (int r = 0; r < run; ++r) {
+        const int c = (warp * run + r) * 32 + lane;
+        const int n = c < ncell ? cells[c] : 0;
+        int incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (c < ncell) cells[c] = carry + incl - n;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) s_tot[warp] = carry;
+    __syncthreads();
+    int before = 0;
+    for (int w = 0; w < warp; ++w) before += s_tot[w];
+    for (int r = 0; r < run; ++r) {
+        const int c = (warp * run + r) * 32 + lane;
+        if (c < ncell) cells[c] += before;
+    }
+}
 
 // one exchange of the row reduction: keep v on the lower lanes and w on the upper ones of
 // each pair `o` apart, adding what the other lane holds of it
@@ -311,10 +340,11 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch *
         const int a = KIND == ATM64_CENTER ? p.atm_apex[item] : p.sorted_of[p.n - 1 - item];
         const SG &g = p.sg[p.sid[a]];
         if (KIND != ATM64_CENTER && warp_uniform(g.atm_simple) != (KIND == ATM64_SIMPLE ? 1 : 0)) continue; // the other instance's
-        const bool ref = KIND == ATM64_WEIGHTED && atm_reference_order(p, g, p.sid[a]);
         const long long e0 = p.atm_off[a];
         const int m = warp_uniform((int)(p.atm_off[a + 1] - e0));
+        if (KIND != ATM64_CENTER && m <= p.atm_min_m) continue; // k_atm64b's
         const double4 xa = p.xs[a];
+        const bool ref = KIND == ATM64_WEIGHTED && atm_reference_order(p, g, p.sid[a]);
         const double *r0a = r0sq + (int)xa.w * ne;
         for (int k = tid; k < ne * NR; k += blockDim.x) yapex[k] = p.Y[(size_t)a * ne * NR + k];
         // types staged together and partner tile: all partners of the apex with as many
@@ -352,31 +382,7 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch *
             __syncthreads();
             for (int k = tid; k < bn; k += blockDim.x) atomicAdd(&cells[cell_of(p.atm_ent[e0 + b0 + k])], 1);
             __syncthreads();
-            {
-                // exclusive scan of the cell counts: a run of 32 cells per warp and step
-                const int run = (ncell / 32 + nw - 1) / nw; // steps per warp
-                int carry = 0;
-                for (int r = 0; r < run; ++r) {
-                    const int c = (warp * run + r) * 32 + lane;
-                    const int n = c < ncell ? cells[c] : 0;
-                    int incl = n;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int u = __shfl_up_sync(0xffffffffu, incl, o);
-                        if (lane >= o) incl += u;
-                    }
-                    if (c < ncell) cells[c] = carry + incl - n;
-                    carry += __shfl_sync(0xffffffffu, incl, 31);
-                }
-                if (lane == 0) s_tot[warp] = carry;
-                __syncthreads();
-                int before = 0;
-                for (int w = 0; w < warp; ++w) before += s_tot[w];
-                for (int r = 0; r < run; ++r) {
-                    const int c = (warp * run + r) * 32 + lane;
-                    if (c < ncell) cells[c] += before;
-                }
-            }
+            atm64_scan(cells, ncell, s_tot);
             __syncthreads();
             for (int k = tid; k < bn; k += blockDim.x) {
                 const int2 ent = p.atm_ent[e0 + b0 + k];

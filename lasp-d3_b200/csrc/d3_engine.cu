@@ -49,6 +49,8 @@ constexpr double K3 = 4.0;
 // floats per (atom, partner type) row of the block-pair ATM table (NR 5 or 7: 12 or 16,
 // whole float4s)
 __host__ __device__ constexpr int atmb_row_floats(int nr) { return 2 * nr + 2; }
+// doubles per row of the YD64 table: Y[NR] D[NR] r0^2 and padding to whole double2 words
+__host__ __device__ constexpr int atm64b_row(int NR) { return 2 * NR + 2; }
 
 // ------------------------------------------------------------------------------------
 // kernel parameter block (passed by value)
@@ -127,7 +129,8 @@ struct KP {
     float *w32, *dw32, *Y32;
     float *YD32;    // [n][ne][2 NR + 2] (block-pair ATM): per partner type the C6 row, r0^2 of
                     // the type pair, the row of the weight derivatives, the atom index bits
-    int atm_min_m;  // k_atm32 takes only apexes with longer lists (the rest: k_atm32b)
+    double *YD64;   // [n][ne][atm64b_row]: the same rows in FP64: Y, D, r0^2
+    int atm_min_m;  // k_atm32 / k_atm64 take only apexes with longer lists (the rest: block pairs)
     int atmb_mcap;  // longest list k_atm32b takes
     int atmb_split; // CTAs of k_atm32b sharing one apex (each a share of its block rows)
     // sharded evaluation: this process computes the two-body and chain-rule terms of the
@@ -537,14 +540,24 @@ __global__ void k_weights(KP p) {
             for (int a = 0; a < NR; ++a) acc += w[a] * C[a * NR + b];
             Yo[b] = acc;
             if (p.precision) p.Y32[((size_t)i * p.ne + tt) * NR + b] = (float)acc;
-            if (p.YD32) {
+            if (p.YD32 || p.YD64) {
                 double dacc = 0.0;
 #pragma unroll
                 for (int a = 0; a < NR; ++a) dacc += dw[a] * C[a * NR + b];
-                float *r = p.YD32 + ((size_t)i * p.ne + tt) * atmb_row_floats(NR);
-                r[b] = (float)acc;
-                r[NR + 1 + b] = (float)dacc;
+                if (p.YD32) {
+                    float *r = p.YD32 + ((size_t)i * p.ne + tt) * atmb_row_floats(NR);
+                    r[b] = (float)acc;
+                    r[NR + 1 + b] = (float)dacc;
+                } else {
+                    double *r = p.YD64 + ((size_t)i * p.ne + tt) * atm64b_row(NR);
+                    r[b] = acc;
+                    r[NR + b] = dacc;
+                }
             }
+        }
+        if (p.YD64) {
+            const double r0 = p.r0ab[tt * p.ne + t];
+            p.YD64[((size_t)i * p.ne + tt) * atm64b_row(NR) + 2 * NR] = r0 * r0;
         }
         if (p.YD32) {
             float *r = p.YD32 + ((size_t)i * p.ne + tt) * atmb_row_floats(NR);
@@ -1012,6 +1025,7 @@ __global__ void k_chain32(KP p, const double *Gd) {
 #include "d3_atm32.cuh"
 #include "d3_atm32b.cuh"
 #include "d3_atm.cuh"
+#include "d3_atm64b.cuh"
 #include "d3_surrogate.cuh"
 
 // ------------------------------------------------------------------------------------
@@ -1275,6 +1289,8 @@ struct Engine {
     DBuf<float> w32, dw32, Y32, YD32;
     DBuf<float4> atmb_scratch;
     DBuf<Atm64Scratch> atm64_scratch;
+    DBuf<Atm64bScratch> atm64b_scratch;
+    DBuf<double> YD64;
     DBuf<long long> atm_off;
     DBuf<int2> atm_ent;
     long long atm_cap = 0;
@@ -1299,7 +1315,7 @@ struct Engine {
         const void *fn = nullptr;
         size_t sm = 0;
         int blocks = 1;
-    } atm_occ_cache[12]; // 0, 2, 4 FP64 ATM, 1, 3 mirror, 5 grouped two-body, 8-11 block-pair ATM
+    } atm_occ_cache[12]; // 0, 2, 4 FP64 ATM, 6, 7 its block pairs, 1, 3 mirror, 5 grouped two-body, 8-11 block-pair ATM
     SurrState surr;
     int shard_rank = 0, shard_world = 0; // set by engine_shard_begin
     int eval_rank = 0, eval_world = 1;   // of the last evaluation
@@ -1324,6 +1340,8 @@ struct Engine {
         YD32.release();
         atmb_scratch.release();
         atm64_scratch.release();
+        atm64b_scratch.release();
+        YD64.release();
         xw_in.release();
         xs.release();
         atm_off.release();
@@ -1905,6 +1923,25 @@ static int apex_split(long long apexes, long long ctas, int most, double setup) 
     return best;
 }
 
+// warps per CTA of the FP64 block-pair kernel, 0 when it is not used: FP32 form, surrogate,
+// the mirror schedule chosen, or where k_atm64 is the faster one: rows of so many types that
+// fewer than eight warps fit the shared memory (k_atm64 stages them type by type), apexes so
+// few that more than four CTAs share one and repeat its sort (16 atoms: 0.38 against 0.62 ms,
+// 32 atoms 1.14 / 1.44, 48 atoms 1.47 / 1.30, 96 atoms 2.65 / 2.12) and short lists (20,000
+// atoms with 18 entries each 1.79 / 2.01 ms, 5,000 with 62 each 0.87 / 0.83)
+static int atm64b_warps(const Engine *e, bool simple = false) {
+    if (!e->use_atm || e->opt.precision || e->opt.atm_schedule != 0 || (e->opt.atm_surrogate && e->surr.loaded)) return 0;
+    if (4 * e->n < (uint64_t)e->dev_sms) return 0;
+    double entries = 0.0; // expected, all apexes together
+    for (size_t k = 0; k < e->sg.size(); ++k)
+        entries += 0.5 * 4.18879020478639 * e->rc_atm * e->rc_atm * e->rc_atm * e->sg[k].natoms * e->sg[k].natoms / std::fabs(e->geoms[k].volume);
+    if (entries < 48.0 * (double)e->n) return 0;
+    const size_t room = 227 * 1024 - ATM64B_STATIC - atm64b_fixed(e->ne, e->nref);
+    const int w = (int)std::min<size_t>(ATM64B_WARPS, room / atm64b_warp(e->ne, e->nref, simple));
+    // (the sort's cells and entry numbers lie in the staging area)
+    return w >= 8 && w * atm64b_warp(e->ne, e->nref, simple) >= (ATM64_CELLS + ATM64B_MCAP) * sizeof(int) ? w : 0;
+}
+
 // CTAs per SM of the FP64 ATM kernel, their shared memory and the splits of an apex
 struct Atm64Shape {
     int ctas, split;
@@ -1976,6 +2013,12 @@ static KP make_kp(Engine *e) {
         const int ctas = e->dev_sms * sh.ctas;
         p.atmb_split = e->opt.atmb_split > 0 ? std::min(e->opt.atmb_split, 64)
                                              : apex_split(std::max(1, p.n), ctas, 16, 0.05);
+    }
+    p.YD64 = nullptr;
+    if (atm64b_warps(e) > 0) {
+        e->YD64.ensure((size_t)e->max_atoms * e->ne * atm64b_row(e->nref));
+        e->atm64b_scratch.ensure((size_t)e->dev_sms);
+        p.YD64 = e->YD64.p;
     }
     if (e->use_atm && !p.precision) {
         const Atm64Shape sh = atm64_shape(e, 1);
@@ -2102,6 +2145,24 @@ static void launch_atm64(Engine *e, const KP &p0, cudaStream_t s, bool center) {
     const void *fns[3] = {(const void *)k_atm64<NR, ATM64_SIMPLE>, (const void *)k_atm64<NR, ATM64_WEIGHTED>,
                           (const void *)k_atm64<NR, ATM64_CENTER>};
     const int cache[3] = {0, 4, 2};
+    const int nwb = center ? 0 : atm64b_warps(e);
+    if (nwb > 0) {
+        // lists up to ATM64B_MCAP entries: block pairs; longer ones below
+        KP q = p;
+        q.atmb_split = apex_split(std::max(1, p.n / p.shard_world), e->dev_sms, 32, 0.02);
+        const void *fnb[2] = {(const void *)k_atm64b<NR, true>, (const void *)k_atm64b<NR, false>};
+        for (int k = 0; k < 2; ++k) { // ATM64_SIMPLE, ATM64_WEIGHTED
+            if (!kind[k]) continue;
+            const int nw = atm64b_warps(e, k == ATM64_SIMPLE);
+            const size_t smb = atm64b_fixed(p.ne, NR) + nw * atm64b_warp(p.ne, NR, k == ATM64_SIMPLE);
+            if (k == 1 && kind[0]) D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
+            atm_occupancy(e, 6 + k, smb, fnb[k]);
+            void *args[] = {(void *)&q, (void *)&e->atm64b_scratch.p};
+            D3_CUDA(cudaLaunchKernel(fnb[k], dim3(e->dev_sms), dim3(32 * nw), args, smb, s));
+        }
+        D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
+        p.atm_min_m = ATM64B_MCAP;
+    }
     for (int k = 0; k < 3; ++k) {
         if (!kind[k]) continue;
         if (k == ATM64_WEIGHTED && kind[ATM64_SIMPLE]) D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
