@@ -2450,7 +2450,7 @@ static void launch_all(Engine *e, const KP &p0, cudaStream_t s, int stage = 0, d
         if (surr) {
             SurrState &S = e->surr;
             sd = surr_desc(S.chan.p, S.L.nch, S.G.p, S.dX.p, S.center.p);
-            k_desc_fwd<NR><<<gw, T, 0, s>>>(p, sd);
+            k_desc_fwd<NR><<<(n + SURR_WARPS - 1) / SURR_WARPS, SURR_WARPS * 32, 0, s>>>(p, sd);
             d3mlp::infer(surr_net(S), S.G.p, S.center.p, n, S.E.p, S.dX.p, e->dev_sms, s);
             D3_CUDA(cudaMemsetAsync(S.napex.p, 0, sizeof(int), s));
             SurrComb c{};
@@ -2475,7 +2475,7 @@ static void launch_all(Engine *e, const KP &p0, cudaStream_t s, int stage = 0, d
         D3_CUDA(cudaEventRecord(ev[4], s));
         if (e->use_atm) {
             launch_atm_triplets<NR>(e, pc, s, surr);
-            if (surr) k_desc_bwd<NR><<<gw, T, 0, s>>>(p, sd);
+            if (surr) k_desc_bwd<NR><<<(n + SURR_WARPS - 1) / SURR_WARPS, SURR_WARPS * 32, 0, s>>>(p, sd);
         }
         D3_CUDA(cudaEventRecord(ev[5], s));
         k_sum_g<<<gb, T, 0, s>>>(p, Gsum);
@@ -2877,9 +2877,9 @@ int engine_surrogate_descriptors(Engine *e, const int *channel_z, int nch, float
         const int T = 256;
         const int gw = (int)(((long long)n * 32 + T - 1) / T);
         if (e->nref == 5)
-            k_desc_fwd<5><<<gw, T, 0, s>>>(p, sd);
+            k_desc_fwd<5><<<(p.n + SURR_WARPS - 1) / SURR_WARPS, SURR_WARPS * 32, 0, s>>>(p, sd);
         else
-            k_desc_fwd<7><<<gw, T, 0, s>>>(p, sd);
+            k_desc_fwd<7><<<(p.n + SURR_WARPS - 1) / SURR_WARPS, SURR_WARPS * 32, 0, s>>>(p, sd);
         k_surr_export<<<gw, T, 0, s>>>(p, S.xG.p, S.xcenter.p, (int)nfeat, G_dev, center_dev, e_atm_dev);
         D3_CUDA(cudaGetLastError());
         D3_CUDA(cudaStreamSynchronize(s));
