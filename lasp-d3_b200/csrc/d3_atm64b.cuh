@@ -20,10 +20,10 @@
 // busy, an FP64 instruction counting twice) and the shared-memory pipe (59 %). Testing every
 // step just before its visit took 186 ms instead of 157.
 // ATM pass on a B200, k_atm64 -> this kernel: 96-atom water box 2.65 -> 2.11 ms, 777 atoms 20.7
-// -> 17.9 ms, 2,000 atoms 50.0 -> 44.3 ms, 20,000-atom box 443 -> 394 ms, batch of 48
-// structures 106 -> 98 ms.
+// -> 17.9 ms, 2,000 atoms 50.0 -> 44.3 ms, 20,000-atom box 443 -> 394 ms (383 with two
+// CTAs per SM), batch of 48 structures 106 -> 98 ms.
 
-constexpr int ATM64B_WARPS = 12;   // warps per CTA at most (168 registers a thread)
+constexpr int ATM64B_WARPS = 12;   // warps per SM at most (168 registers a thread)
 constexpr int ATM64B_MCAP = 4096;  // longest list (longer ones: k_atm64)
 constexpr int ATM64B_NACC = 8;     // accumulators per entry: E, dE/dCN, force, virial coefficient
 constexpr int ATM64B_STATIC = 2560;

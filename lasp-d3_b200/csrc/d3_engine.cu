@@ -1923,23 +1923,34 @@ static int apex_split(long long apexes, long long ctas, int most, double setup) 
     return best;
 }
 
-// warps per CTA of the FP64 block-pair kernel, 0 when it is not used: FP32 form, surrogate,
-// the mirror schedule chosen, or where k_atm64 is the faster one: rows of so many types that
+// Shape of the FP64 block-pair kernel; no warps when it is not used: FP32 form, surrogate, the
+// mirror schedule chosen, or where k_atm64 is the faster one: rows of so many types that
 // fewer than eight warps fit the shared memory (k_atm64 stages them type by type), apexes so
 // few that more than four CTAs share one and repeat its sort (16 atoms: 0.38 against 0.62 ms,
 // 32 atoms 1.14 / 1.44, 48 atoms 1.47 / 1.30, 96 atoms 2.65 / 2.12) and short lists (20,000
-// atoms with 18 entries each 1.79 / 2.01 ms, 5,000 with 62 each 0.87 / 0.83)
-static int atm64b_warps(const Engine *e, bool simple = false) {
-    if (!e->use_atm || e->opt.precision || e->opt.atm_schedule != 0 || (e->opt.atm_surrogate && e->surr.loaded)) return 0;
-    if (4 * e->n < (uint64_t)e->dev_sms) return 0;
+// atoms with 18 entries each 1.79 / 2.01 ms, 5,000 with 62 each 0.87 / 0.83).
+// Two CTAs per SM for weight-free structures, where the set-up of one apex overlaps the
+// visits of another (8,000 atoms 157 -> 154 ms, 4,000 atoms of short lists 2.93 -> 2.50 ms);
+// one for the others, whose virial carries leave room for fewer warps in halves (2,000 atoms
+// 44.2 against 46.2 ms, batch of 48 structures 98 against 108 ms).
+struct Atm64bShape {
+    int warps, ctas; // per CTA, per SM
+};
+static Atm64bShape atm64b_shape(const Engine *e, bool simple) {
+    if (!e->use_atm || e->opt.precision || e->opt.atm_schedule != 0 || (e->opt.atm_surrogate && e->surr.loaded)) return {0, 1};
+    if (4 * e->n < (uint64_t)e->dev_sms) return {0, 1};
     double entries = 0.0; // expected, all apexes together
     for (size_t k = 0; k < e->sg.size(); ++k)
         entries += 0.5 * 4.18879020478639 * e->rc_atm * e->rc_atm * e->rc_atm * e->sg[k].natoms * e->sg[k].natoms / std::fabs(e->geoms[k].volume);
-    if (entries < 48.0 * (double)e->n) return 0;
-    const size_t room = 227 * 1024 - ATM64B_STATIC - atm64b_fixed(e->ne, e->nref);
-    const int w = (int)std::min<size_t>(ATM64B_WARPS, room / atm64b_warp(e->ne, e->nref, simple));
-    // (the sort's cells and entry numbers lie in the staging area)
-    return w >= 8 && w * atm64b_warp(e->ne, e->nref, simple) >= (ATM64_CELLS + ATM64B_MCAP) * sizeof(int) ? w : 0;
+    if (entries < 48.0 * (double)e->n) return {0, 1};
+    const size_t per = atm64b_warp(e->ne, e->nref, simple);
+    for (int ctas = simple ? 2 : 1; ctas >= 1; --ctas) {
+        const size_t room = std::min<size_t>(227 * 1024, 228 * 1024 / ctas - 1024) - ATM64B_STATIC - atm64b_fixed(e->ne, e->nref);
+        const int w = (int)std::min<size_t>(ATM64B_WARPS / ctas, room / per);
+        // (the sort's cells and entry numbers lie in the staging area)
+        if (w * ctas >= 8 && w * per >= (ATM64_CELLS + ATM64B_MCAP) * sizeof(int)) return {w, ctas};
+    }
+    return {0, 1};
 }
 
 // CTAs per SM of the FP64 ATM kernel, their shared memory and the splits of an apex
@@ -2015,9 +2026,12 @@ static KP make_kp(Engine *e) {
                                              : apex_split(std::max(1, p.n), ctas, 16, 0.05);
     }
     p.YD64 = nullptr;
-    if (atm64b_warps(e) > 0) {
+    const Atm64bShape shb[2] = {atm64b_shape(e, true), atm64b_shape(e, false)};
+    if (shb[0].warps > 0 || shb[1].warps > 0) {
+        bool simple = false;
+        for (const SG &q : e->sg) simple |= q.atm_simple != 0;
         e->YD64.ensure((size_t)e->max_atoms * e->ne * atm64b_row(e->nref));
-        e->atm64b_scratch.ensure((size_t)e->dev_sms);
+        e->atm64b_scratch.ensure((size_t)e->dev_sms * (simple ? shb[0].ctas : 1));
         p.YD64 = e->YD64.p;
     }
     if (e->use_atm && !p.precision) {
@@ -2145,20 +2159,20 @@ static void launch_atm64(Engine *e, const KP &p0, cudaStream_t s, bool center) {
     const void *fns[3] = {(const void *)k_atm64<NR, ATM64_SIMPLE>, (const void *)k_atm64<NR, ATM64_WEIGHTED>,
                           (const void *)k_atm64<NR, ATM64_CENTER>};
     const int cache[3] = {0, 4, 2};
-    const int nwb = center ? 0 : atm64b_warps(e);
-    if (nwb > 0) {
+    const Atm64bShape shapes[2] = {atm64b_shape(e, true), atm64b_shape(e, false)}; // ATM64_SIMPLE, ATM64_WEIGHTED
+    if (!center && (!kind[0] || shapes[0].warps > 0) && (!kind[1] || shapes[1].warps > 0)) {
         // lists up to ATM64B_MCAP entries: block pairs; longer ones below
         KP q = p;
-        q.atmb_split = apex_split(std::max(1, p.n / p.shard_world), e->dev_sms, 32, 0.02);
         const void *fnb[2] = {(const void *)k_atm64b<NR, true>, (const void *)k_atm64b<NR, false>};
-        for (int k = 0; k < 2; ++k) { // ATM64_SIMPLE, ATM64_WEIGHTED
+        for (int k = 0; k < 2; ++k) {
             if (!kind[k]) continue;
-            const int nw = atm64b_warps(e, k == ATM64_SIMPLE);
+            const int nw = shapes[k].warps, grid_b = e->dev_sms * shapes[k].ctas;
+            q.atmb_split = apex_split(std::max(1, p.n / p.shard_world), grid_b, 32, 0.02);
             const size_t smb = atm64b_fixed(p.ne, NR) + nw * atm64b_warp(p.ne, NR, k == ATM64_SIMPLE);
             if (k == 1 && kind[0]) D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
             atm_occupancy(e, 6 + k, smb, fnb[k]);
             void *args[] = {(void *)&q, (void *)&e->atm64b_scratch.p};
-            D3_CUDA(cudaLaunchKernel(fnb[k], dim3(e->dev_sms), dim3(32 * nw), args, smb, s));
+            D3_CUDA(cudaLaunchKernel(fnb[k], dim3(grid_b), dim3(32 * nw), args, smb, s));
         }
         D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
         p.atm_min_m = ATM64B_MCAP;

@@ -62,3 +62,16 @@ def test_lists_on_both_sides_of_the_capacity():
     assert a[3] == b[3]
     assert abs(a[0] - b[0]) <= 1e-9 * abs(b[0])
     assert np.abs(a[1] - b[1]).max() <= 1e-7 and np.abs(a[2] - b[2]).max() <= 1e-7
+
+
+@pytest.mark.parametrize("mix,ext", [(ONE, False), (ONE, True), (SEVEN, False), (SEVEN, True)])
+def test_weight_free_boxes_of_one_and_many_types(mix, ext):
+    """Both ends of the shared-memory rule in weight-free boxes (two CTAs per SM, one, or the
+    other schedule)."""
+    s = box(700, 0.02, mix, seed=9)
+    a, b = evaluate(s, 20.0, ext, False, 0), evaluate(s, 20.0, ext, False, 1)
+    r = oracle.compute(s["pos"], s["Z"], s["cell"], rc=50.0, rc_cn=25.0, rc_atm=20.0, extended=ext, c6_mode=1)
+    for e, f, st, visits in (a, b):
+        assert abs(e - r["energy"]) <= 1e-9 * abs(r["energy"])
+        assert np.abs(f - r["forces"]).max() <= 1e-7 and np.abs(st - r["stress"]).max() <= 1e-7
+    assert a[3] == b[3]
