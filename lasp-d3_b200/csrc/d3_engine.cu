@@ -1890,6 +1890,18 @@ static const void *pairs_kernel(const Engine *e) {
     return f64 ? (const void *)k_twobody_g<7, true> : (const void *)k_twobody_g<7, false>;
 }
 
+// Lets a kernel take all the dynamic shared memory the device has. The limit belongs to the
+// function, not to the handle: with each handle setting its own size, a handle of few element
+// types took the limit below what another handle's next launch needs.
+static void allow_smem(const void *fn) {
+    cudaFuncAttributes at;
+    int dev = 0, most = 0;
+    D3_CUDA(cudaFuncGetAttributes(&at, fn));
+    D3_CUDA(cudaGetDevice(&dev));
+    D3_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    D3_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes));
+}
+
 // CTAs per SM of the grouped two-body kernel (attribute and query cached, so that an
 // evaluation inside a graph capture makes no such call)
 static int pairs_occupancy(Engine *e) {
@@ -1897,7 +1909,7 @@ static int pairs_occupancy(Engine *e) {
     const void *fn = pairs_kernel(e);
     const size_t sm = pairs_smem(e);
     if (c.fn == fn && c.sm == sm) return c.blocks;
-    D3_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    allow_smem(fn);
     int blocks = 0;
     D3_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, PAIRS_WARPS * 32, sm));
     c.fn = fn;
@@ -2122,7 +2134,7 @@ static const void *blockpair_fn(bool fine) {
 static int atm_occupancy(Engine *e, int which, size_t sm, const void *fn) {
     auto &c = e->atm_occ_cache[which];
     if (c.fn == fn && c.sm == sm) return c.blocks;
-    D3_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    allow_smem(fn);
     int blocks = 0;
     D3_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, ATM_THREADS, sm));
     c.fn = fn;
