@@ -331,7 +331,7 @@ def engine_arm(args, world, rank, local):
         tfile = os.path.join(ROOT, "profiles", "ncu_traffic.json")
         if os.path.exists(tfile) and args.system == "triclinic" and n == N_ATOMS and table == TABLE_5REF:
             traffic = json.load(open(tfile)).get("atm_fp64_bytes_per_launch" if fp64 else "atm_fp32_bytes_per_launch")
-        kernel = ("k_atm (ATM triplets, FP64)" if fp64 else
+        kernel = ("k_atm64b + k_atm64 (ATM triplets, FP64; block pairs, lists beyond their capacity and small cases by rows)" if fp64 else
                   "k_atm32b + k_atm32 (ATM triplets, FP32 arithmetic; block pairs, packed f32x2 pairs of visits; lists beyond the per-launch block-pair capacity mirrored)")
         algorithmic = "%d in-range triplets x %d FLOP per launch" % (triplets, ATM_FLOP_PER_TRIPLET)
     else:

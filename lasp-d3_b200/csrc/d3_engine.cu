@@ -19,7 +19,7 @@
 //                           their CN derivative
 //   Y[n][ne][NR]            y_{i,t}[b] = sum_a w_i[a] C6ref[t_i][t][a][b]
 //   per-atom energy / dE/dCN / force / virial partials of each pass
-//   atm_off[n+1], atm_ent[] rc_ATM half list (j <= a in caller order), CSR
+//   atm_off[n+1], atm_ent[] rc_ATM half list (entries before the apex, atm_before), CSR
 #include "d3_engine.h"
 
 #include <cuda_runtime.h>
@@ -2550,7 +2550,9 @@ int engine_launches_per_eval(const Engine *e) {
     const int pairs = pairs_grouped(e) ? (e->use_atm ? 5 : 4) : 0;
     if (!e->use_atm) return 12 + pairs;
     if (e->opt.atm_surrogate && e->surr.loaded) return 20 + pairs;
-    return (blockpair_warps(e) > 0 ? 17 : 16) + pairs;
+    // block pairs and, behind them, the lists too long for them
+    const bool blocks = blockpair_warps(e) > 0 || atm64b_shape(e, true).warps > 0 || atm64b_shape(e, false).warps > 0;
+    return (blocks ? 17 : 16) + pairs;
 }
 
 // Accuracy check of the Newton-refined helpers used by the ATM kernel against CUDA's

@@ -46,10 +46,10 @@ struct Options {
                                    // FP64 weights, dE/dCN and reductions (precision form)
     // tunables (set by the autotuner or the caller)
     double bin_divisor = 6.0;      // bin width = smallest cutoff / bin_divisor
-    int atm_tile = 0;              // ATM partner tile entries (0: largest that fits, <= 128)
+    int atm_tile = 0;              // ATM partner tile entries (0: largest that fits; k_atm32: <= 128)
     int atm_ctas_per_sm = 0;       // persistent ATM CTAs per SM (0: occupancy limit)
     bool atm_surrogate = false;    // learned ATM surrogate with exact fallback (needs a model)
-    int atm_schedule = 0;          // precision-form ATM: 0 block pairs (each triplet once),
+    int atm_schedule = 0;          // ATM: 0 block pairs (each triplet once; FP64: by rule),
                                    // 1 mirror-symmetric full square (each triplet twice)
     long long atm_list_capacity = 0; // ATM half-list entries to allocate (0: estimate from the
                                      // density); a synchronous evaluation regrows on overflow
