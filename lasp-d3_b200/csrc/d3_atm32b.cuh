@@ -28,7 +28,7 @@
 //     virial sum v_e (x) F_e, plus in the weighted form the corrections for the visits
 //     whose energy weight w differs from the force weight wf.
 // With f1, f2, f3 the force scalars of sides a-x, a-y, x-y of a triplet (mirror symmetry of
-// k_atm: f2 of visit (x, y) is f1 of the mirrored visit), the quantities per entry are
+// k_atm32: f2 of visit (x, y) is f1 of the mirrored visit), the quantities per entry are
 //   SE = sum w E, SD = sum w E lam_{e,other}, F = sum wf ((f_apex-side + f3) v_e - f3 v_other);
 // x lanes keep F as SF = sum wf (f_apex-side + f3) and W = sum wf f3 v_other (v_x is fixed
 // along the row), y sums carry -F itself (five travelling quantities).
