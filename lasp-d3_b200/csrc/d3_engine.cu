@@ -146,7 +146,7 @@ struct KP {
     int *anyshift;           // per structure: some atom was given outside the cell
     unsigned int *span;      // per structure and lattice direction: extent of the positions as
                              // given (SPAN0 - floor, SPAN0 + ceil of the fractional
-                             // coordinates x 65536, each the largest over the atoms)
+                             // coordinates x SPAN_SCALE, each the largest over the atoms)
     int atm_ref_order;       // 1: ATM lists in the reference's order (diagnostics)
     const int4 *srows;
     int nsrow;
@@ -163,7 +163,10 @@ __device__ __forceinline__ int floordiv(int a, int b) {
     return q;
 }
 
+// (coordinates up to FRAC_MAX, all that k_bin accepts, keep the extents within 31 bits)
 constexpr unsigned int SPAN0 = 1u << 30;
+constexpr double FRAC_MAX = 1.0e6, SPAN_SCALE = 1024.0;
+static_assert(FRAC_MAX * SPAN_SCALE < (double)SPAN0, "extents of the farthest atoms");
 
 // Order of the ATM half lists. A triplet of lattice points is visited from the apex that
 // comes last in a translation-invariant order: by height along the third lattice vector
@@ -183,7 +186,7 @@ __device__ __forceinline__ bool atm_reference_order(const KP &p, const SG &g, in
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const int extent = (int)(p.span[6 * sid + 2 * k] - SPAN0) + (int)(p.span[6 * sid + 2 * k + 1] - SPAN0);
-        cut |= (int)floor(extent * (1.0 / 65536.0) + g.ratm_frac[k] + 1e-6) > g.half[k];
+        cut |= (int)floor(extent * (1.0 / SPAN_SCALE) + g.ratm_frac[k] + 1e-6) > g.half[k];
     }
     return cut;
 }
@@ -323,13 +326,13 @@ __global__ void k_bin(KP p) {
     bool bad = !(isfinite(x) && isfinite(y) && isfinite(z));
     for (int k = 0; k < 3; ++k) {
         double f = x * g.inv[0 * 3 + k] + y * g.inv[1 * 3 + k] + z * g.inv[2 * 3 + k];
-        if (bad || fabs(f) > 1.0e6) {
+        if (bad || fabs(f) > FRAC_MAX) {
             bad = true;
             f = 0.0;
         }
         double fl = floor(f);
         s[k] = (int)fl;
-        const double q = fmin(fmax(f, -16000.0), 16000.0) * 65536.0;
+        const double q = f * SPAN_SCALE;
         ext[2 * k] = SPAN0 - (int)floor(q);
         ext[2 * k + 1] = SPAN0 + (int)ceil(q);
         int bk = (int)((f - fl) * g.nb[k]);
