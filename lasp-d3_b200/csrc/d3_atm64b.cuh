@@ -297,9 +297,11 @@ __global__ void __launch_bounds__(ATM64B_WARPS * 32, 1) k_atm64b(KP p, Atm64bScr
                     yY = fma(f3, vy, fma(-f23, A0.y, yY));
                     yZ = fma(f3, vz, fma(-f23, A1.x, yZ));
                 }
-                // lane L holds the sums of B[(L + at) mod 32]
+                // lane L holds the sums of B[(L + at) mod 32] (no bit set: not visited; a triplet
+                // may have forces and no energy)
                 const int e = 32 * B + ((lane + at) & 31);
-                if (e < m && yE != 0.0) {
+                const long long any = __double_as_longlong(yE) | __double_as_longlong(yX) | __double_as_longlong(yY) | __double_as_longlong(yZ);
+                if (e < m && any != 0) {
                     double *o = acc[e];
                     atomicAdd(o, yE);
                     atomicAdd(o + 1, yD);
