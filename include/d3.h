@@ -196,7 +196,10 @@ int d3_fetch_results(d3_handle_t *handle, double *energies, double *forces, doub
    evaluation: [0] wrap+bin, [1] CN + C6 weights, [2] two-body, [3] ATM list,
    [4] ATM triplets, [5] chain rule, [6] finalize; returns the number written.
    counters (may be NULL) receives 4 values: ATM in-range triplet visits (two per
-   triplet), two-body in-range ordered pairs, CN in-range ordered pairs, 0. */
+   triplet of the reference's enumeration), two-body in-range ordered pairs, CN in-range
+   ordered pairs, 0. In cells shorter than the ATM cutoff the reference visits triplets with
+   repeated atoms more than once; counting those synchronises the device and takes about a
+   millisecond, with NULL nothing is counted. */
 int d3_pass_times(d3_handle_t *handle, float *ms, int cap, uint64_t *counters);
 
 /* Number of kernels one evaluation launches. */

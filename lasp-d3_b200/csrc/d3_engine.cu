@@ -68,6 +68,7 @@ struct SG {
     int stcb_off, stcb_n;     // CN / chain-rule stencil of the same blocks
     int stab_off, stab_n;     // rc_ATM stencil of the same blocks (ATM half lists)
     int atm_simple;           // every cell height > 2 rc_ATM: no atom twice in an ATM list
+    int atm_images[3];        // lattice vectors within rc_ATM span at most +- this many cells
     double ratm_frac[3];      // rc_ATM over the cell heights
 };
 
@@ -1321,11 +1322,15 @@ struct Engine {
     } atm_occ_cache[12]; // 0, 2, 4 FP64 ATM, 6, 7 its block pairs, 1, 3 mirror, 5 grouped two-body, 8-11 block-pair ATM
     SurrState surr;
     int shard_rank = 0, shard_world = 0; // set by engine_shard_begin
-    int eval_rank = 0, eval_world = 1;   // of the last evaluation
-    Options eval_opt{};                  // its options
-    bool eval_current = false;           // the atoms and geometry on the device are still its own
-    bool extra_known = false;            // extra_visits holds for it
-    unsigned long long extra_visits = 0;
+    // of the last evaluation, for its diagnostics: shard, options, atom count (0: none yet)
+    // and geometry (in sg, geoms, stencil_rows until a new one takes their place)
+    int eval_rank = 0, eval_world = 1;
+    Options eval_opt{};
+    uint64_t eval_n = 0;
+    bool eval_geometry_moved = false;
+    std::vector<SG> eval_sg;
+    std::vector<CellGeom> eval_geoms;
+    std::vector<int4> eval_rows;
 
     ~Engine() {
         DBuf<double> *ds[] = {&t_cnref, &t_c6, &t_r0, &t_rcov, &t_r2r4, &t_pairA, &pos_in, &cn, &w, &dw, &Y, &e2,
@@ -1568,7 +1573,8 @@ Engine *engine_create(const uint16_t *elements, uint64_t n_elements, uint64_t ma
         e->sg_dev.ensure(max_structs);
         e->out.ensure(10 * max_structs + 3 * N);
         e->status.ensure(1);
-        e->counters.ensure(5);
+        e->counters.ensure(4);
+        e->anyshift.ensure(7 * max_structs); // flag, then the six extents, per structure
         for (auto &x : e->ev) D3_CUDA(cudaEventCreate(&x));
         e->host_out.resize(10 * max_structs + 3 * N);
         return e;
@@ -1624,7 +1630,6 @@ static std::vector<int> map_types(const Engine *e, const uint16_t *Z, uint64_t n
 // stencils; uploads the records, the stencil rows and the per-atom structure index.
 static void build_structures(Engine *e, int nstruct, const uint64_t *counts, const double *cells,
                              const float *cells_f) {
-    e->eval_current = false;
     std::vector<SG> sg(nstruct);
     std::vector<CellGeom> geoms(nstruct);
     std::vector<int4> rows, srow;
@@ -1648,7 +1653,10 @@ static void build_structures(Engine *e, int nstruct, const uint64_t *counts, con
         // a nonzero lattice vector is at least as long as the smallest height, so with every
         // height above 2 rc_ATM two images of one atom never lie within rc_ATM of an apex
         r.atm_simple = std::min(g.height[0], std::min(g.height[1], g.height[2])) > 2.0 * e->rc_atm * (1.0 + 1e-9);
-        for (int i = 0; i < 3; ++i) r.ratm_frac[i] = e->use_atm ? e->rc_atm / g.height[i] : 0.0;
+        for (int i = 0; i < 3; ++i) {
+            r.ratm_frac[i] = e->use_atm ? e->rc_atm / g.height[i] : 0.0;
+            r.atm_images[i] = (int)std::min(std::floor(r.ratm_frac[i] * (1.0 + 1e-9)), 1024.0);
+        }
         int64_t mcb[3];
         r.box_mode = reference_box(cells_f + 9 * k, e->rc_f, e->rc_cn_f, mcb) ? 1 : 0;
         for (int i = 0; i < 3; ++i) r.half[i] = (int)(mcb[i] / 2);
@@ -1697,6 +1705,12 @@ static void build_structures(Engine *e, int nstruct, const uint64_t *counts, con
                 srow.push_back(make_int4(k, by, bz, std::min(gy, r.nb[1] - by) | (std::min(gz, r.nb[2] - bz) << 8)));
         sid.insert(sid.end(), counts[k], k);
     }
+    if (e->eval_n > 0 && !e->eval_geometry_moved) {
+        e->eval_sg.swap(e->sg);
+        e->eval_geoms.swap(e->geoms);
+        e->eval_rows.swap(e->stencil_rows);
+        e->eval_geometry_moved = true;
+    }
     e->sg = sg;
     e->geoms = geoms;
     e->counts.assign(counts, counts + nstruct);
@@ -1713,7 +1727,6 @@ static void build_structures(Engine *e, int nstruct, const uint64_t *counts, con
         D3_CUDA(cudaMemcpy(e->srows.p, srow.data(), sizeof(int4) * srow.size(), cudaMemcpyHostToDevice));
     e->groups.ensure(e->group_bound);
     e->gctl.ensure(6); // [0] groups, [1..5] work counters: CN, two-body, chain, ATM list count, fill
-    e->anyshift.ensure(7 * (size_t)std::max(1, nstruct)); // flag, then the six extents, per structure
     e->nstruct = nstruct;
     e->nbins_total = bin_base;
     e->sg_dev.ensure(nstruct);
@@ -1738,7 +1751,6 @@ int engine_set_atoms(Engine *e, const double *pos_bohr, const uint16_t *Z, uint6
         D3_CUDA(cudaMemcpyAsync(e->type_in.p, types.data(), sizeof(int) * n, cudaMemcpyHostToDevice, e->stream));
         D3_CUDA(cudaStreamSynchronize(e->stream));
         const bool recount = e->n != n;
-        if (recount) e->eval_current = false;
         e->n = n;
         e->atoms_set = true;
         if (e->cell_set && (recount || e->nstruct != 1)) {
@@ -1790,7 +1802,6 @@ int engine_set_batch(Engine *e, uint64_t nstruct, const uint64_t *counts, const 
         D3_CUDA(cudaMemcpyAsync(e->pos_in.p, pos_bohr, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, e->stream));
         D3_CUDA(cudaMemcpyAsync(e->type_in.p, types.data(), sizeof(int) * n, cudaMemcpyHostToDevice, e->stream));
         D3_CUDA(cudaStreamSynchronize(e->stream));
-        e->eval_current = false;
         e->n = n;
         e->atoms_set = true;
         e->cell_set = true;
@@ -2227,65 +2238,56 @@ static d3mlp::Net surr_net(const SurrState &S) {
     return net;
 }
 
-// Triplets that the reference's enumeration visits more than once: with two images of an
-// atom of larger caller index than the third it takes either image as the apex, with three
-// images of one atom each. Counts the additional visits of the lists in the engine's order
-// (only asked for with the work counters), one CTA per apex.
-__global__ void k_atm_extra_visits(KP p, unsigned long long *extra) {
-    const int a = blockIdx.x;
-    const int sid = p.sid[a];
+// Additional visits of the reference's enumeration, for the work counters. It takes a triplet
+// with two images of an atom r and an atom o of smaller caller index from either image, and
+// one with three images of an atom from each. The lists in the engine's order hold every
+// pair of atoms within rc_ATM once, and seen from the pair {o, r}, r of the larger index,
+// the triplets with another image of r are the lattice vectors L within rc_ATM that leave
+// r + L within rc_ATM of o; over all pairs each such triplet is found twice, one with three
+// images of an atom three times. The sum counts 3 and 4 for the two kinds: six times the
+// visits. One row of CTAs per apex.
+constexpr int REPEATS_THREADS = 128, REPEATS_VECTORS = 512;
+__global__ void __launch_bounds__(REPEATS_THREADS) k_atm_repeats(KP p, unsigned long long *sum) {
+    __shared__ double3 vec[REPEATS_VECTORS];
+    __shared__ int nvec;
+    const int a = blockIdx.x, sid = p.sid[a];
     const SG &g = p.sg[sid];
-    if (g.atm_simple || atm_reference_order(p, g, sid) || p.atm_off[p.n] > p.atm_cap) return;
-    const long long e0 = p.atm_off[a];
-    const int m = (int)(p.atm_off[a + 1] - e0);
+    if (atm_reference_order(p, g, sid)) return;
+    const int kx = g.atm_images[0], ky = g.atm_images[1], kz = g.atm_images[2];
+    const int wx = 2 * kx + 1, wy = 2 * ky + 1;
+    const long long box = (long long)wx * wy * (2 * kz + 1);
+    if (box == 1) return;
+    const long long e0 = p.atm_off[a], e1 = p.atm_off[a + 1];
     const double4 xa = p.xs[a];
-    auto pos = [&](int k, int &j) {
-        const int2 ent = p.atm_ent[e0 + k];
-        j = ent.x;
-        const double4 xj = p.xs[j];
-        double sx, sy, sz;
-        image_vec(g, sext8(ent.y & 0xff), sext8((ent.y >> 8) & 0xff), sext8((ent.y >> 16) & 0xff), sx, sy, sz);
-        return make_double3(xj.x + sx - xa.x, xj.y + sy - xa.y, xj.z + sz - xa.z);
-    };
-    unsigned long long more = 0;
-    for (int x = threadIdx.x; x < m; x += blockDim.x) {
-        int jx;
-        const double3 v = pos(x, jx);
-        for (int y = 0; y < x; ++y) {
-            const int jy = p.atm_ent[e0 + y].x;
-            if (jx != jy && jx != a && jy != a) continue;
-            int j;
-            const double3 u = pos(y, j);
-            const double rx = v.x - u.x, ry = v.y - u.y, rz = v.z - u.z;
-            const double d3 = fma(rx, rx, fma(ry, ry, rz * rz));
-            if (d3 > p.ratm2 || d3 < 1e-12) continue;
-            if (jx == jy && jx == a)
-                more += 2;
-            else { // the repeated atom and the other one
-                const int r = jx == jy ? jx : a, o = jx == jy ? a : (jx == a ? jy : jx);
-                more += p.orig[r] > p.orig[o] ? 1 : 0;
+    unsigned long long six = 0;
+    for (long long c0 = 0; c0 < box; c0 += REPEATS_VECTORS) {
+        __syncthreads();
+        if (threadIdx.x == 0) nvec = 0;
+        __syncthreads();
+        for (long long c = c0 + threadIdx.x; c < min(box, c0 + REPEATS_VECTORS); c += blockDim.x) {
+            double3 v;
+            image_vec(g, (int)(c % wx) - kx, (int)(c / wx % wy) - ky, (int)(c / wx / wy) - kz, v.x, v.y, v.z);
+            const double d2 = v.x * v.x + v.y * v.y + v.z * v.z;
+            if (d2 <= p.ratm2 && d2 >= 1e-12) vec[atomicAdd(&nvec, 1)] = v;
+        }
+        __syncthreads();
+        for (long long k = e0 + blockIdx.y * REPEATS_THREADS + threadIdx.x; k < e1; k += (long long)gridDim.y * REPEATS_THREADS) {
+            const int2 ent = p.atm_ent[k];
+            const double4 xj = p.xs[ent.x];
+            double sx, sy, sz;
+            image_vec(g, sext8(ent.y & 0xff), sext8((ent.y >> 8) & 0xff), sext8((ent.y >> 16) & 0xff), sx, sy, sz);
+            const double rx = xj.x + sx - xa.x, ry = xj.y + sy - xa.y, rz = xj.z + sz - xa.z;
+            int found = 0;
+            for (int i = 0; i < nvec; ++i) {
+                const double x = rx + vec[i].x, y = ry + vec[i].y, z = rz + vec[i].z;
+                const double d2 = x * x + y * y + z * z;
+                found += d2 <= p.ratm2 && d2 >= 1e-12 ? 1 : 0;
             }
+            six += (ent.x == a ? 4u : 3u) * (unsigned long long)found;
         }
     }
-    for (int o = 16; o > 0; o >>= 1) more += __shfl_xor_sync(0xffffffffu, more, o);
-    if ((threadIdx.x & 31) == 0 && more) atomicAdd(extra, more);
-}
-
-// additional visits of the last evaluation's triplets in the reference's enumeration
-static unsigned long long engine_extra_visits(Engine *e) {
-    if (e->extra_known) return e->extra_visits;
-    bool weighted = false;
-    for (const SG &q : e->sg) weighted |= !q.atm_simple;
-    unsigned long long n = 0;
-    if (e->use_atm && weighted && e->eval_current && !(e->opt.atm_surrogate && e->surr.loaded)) {
-        KP p = make_kp(e);
-        unsigned long long *d = e->counters.p + 4;
-        D3_CUDA(cudaMemset(d, 0, sizeof(*d)));
-        k_atm_extra_visits<<<p.n, 128>>>(p, d);
-        D3_CUDA(cudaGetLastError());
-        D3_CUDA(cudaMemcpy(&n, d, sizeof(*d), cudaMemcpyDeviceToHost));
-    }
-    return n;
+    for (int o = 16; o > 0; o >>= 1) six += __shfl_xor_sync(0xffffffffu, six, o);
+    if ((threadIdx.x & 31) == 0 && six) atomicAdd(sum, six);
 }
 
 // ATM half lists of every apex (of the flagged ones in centre mode)
@@ -2353,41 +2355,162 @@ static void launch_atm_triplets(Engine *e, const KP &p0, cudaStream_t s, bool su
     }
 }
 
+// rebuilds the bin counts of an evaluation from its atoms' bins
+__global__ void k_count_bins(const int *bin_s, int *cnt, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) atomicAdd(&cnt[bin_s[i]], 1);
+}
+
+// The lists of the last evaluation again, for its diagnostics. Everything written is the
+// pass's own, and what it reads is what the evaluation left of its atoms (binned order,
+// weights) and the geometry it ran with: the handle's lists, sums, status and counters stay,
+// whatever was set since.
+struct EvalLists {
+    DBuf<double> sums;
+    DBuf<long long> off;
+    DBuf<int> cnt, bins, work;
+    DBuf<int2> ent;
+    DBuf<unsigned int> status;
+    DBuf<unsigned long long> repeats;
+    DBuf<SG> sg;
+    DBuf<int4> rows;
+    double *ea = nullptr, *ga = nullptr, *fa = nullptr, *va = nullptr; // apex shares
+    ~EvalLists() {
+        sums.release();
+        off.release();
+        cnt.release();
+        bins.release();
+        work.release();
+        ent.release();
+        status.release();
+        repeats.release();
+        sg.release();
+        rows.release();
+    }
+};
+
+// the options, atom count and geometry of the last evaluation, while a pass over it runs
+struct EvalScope {
+    Engine *e;
+    Options opt;
+    uint64_t n;
+    explicit EvalScope(Engine *eng) : e(eng), opt(eng->opt), n(eng->n) {
+        e->opt = e->eval_opt;
+        e->n = e->eval_n;
+        swap();
+    }
+    ~EvalScope() {
+        e->opt = opt;
+        e->n = n;
+        swap();
+    }
+    void swap() {
+        if (!e->eval_geometry_moved) return;
+        e->sg.swap(e->eval_sg);
+        e->geoms.swap(e->eval_geoms);
+        e->stencil_rows.swap(e->eval_rows);
+    }
+};
+
+// within an EvalScope, the device idle: lists in the reference's order (entries j <= a in
+// caller order) or the engine's
+static KP eval_lists(Engine *e, EvalLists &r, bool ref_order, cudaStream_t s) {
+    const size_t n = e->n;
+    const int T = 256, nbins = e->sg.back().bin_base + e->sg.back().nbins;
+    r.off.ensure(n + 1);
+    r.cnt.ensure(n);
+    r.bins.ensure(2 * (size_t)nbins + 1);
+    r.work.ensure(1);
+    r.status.ensure(1);
+    r.sg.ensure(e->sg.size());
+    r.rows.ensure(e->stencil_rows.size());
+    D3_CUDA(cudaMemcpyAsync(r.sg.p, e->sg.data(), sizeof(SG) * e->sg.size(), cudaMemcpyHostToDevice, s));
+    D3_CUDA(cudaMemcpyAsync(r.rows.p, e->stencil_rows.data(), sizeof(int4) * e->stencil_rows.size(), cudaMemcpyHostToDevice, s));
+    D3_CUDA(cudaMemsetAsync(r.bins.p, 0, sizeof(int) * nbins, s));
+    KP p = make_kp(e);
+    p.shard_rank = e->eval_rank;
+    p.shard_world = e->eval_world;
+    p.atm_ref_order = ref_order ? 1 : 0;
+    p.counters = nullptr;
+    p.nstruct = (int)e->sg.size();
+    p.span = reinterpret_cast<unsigned int *>(e->anyshift.p + e->sg.size());
+    p.sg = r.sg.p;
+    p.stencils = r.rows.p;
+    p.bin_start = r.bins.p + nbins;
+    p.gslices = 0; // lists by the per-apex kernel, which needs no groups
+    p.work = r.work.p;
+    p.status = r.status.p;
+    p.atm_cnt = r.cnt.p;
+    p.atm_off = r.off.p;
+    k_count_bins<<<(int)((n + T - 1) / T), T, 0, s>>>(p.bin_s, r.bins.p, (int)n);
+    k_scan<int, int><<<1, 1024, 0, s>>>(r.bins.p, p.bin_start, nbins);
+    const int gw = (int)((n * 32 + T - 1) / T);
+    k_atm_list<false><<<gw, T, 0, s>>>(p);
+    k_scan<long long, int><<<1, 1024, 0, s>>>(p.atm_cnt, p.atm_off, (int)n);
+    long long need = 0;
+    D3_CUDA(cudaMemcpyAsync(&need, r.off.p + n, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    D3_CUDA(cudaStreamSynchronize(s));
+    r.ent.ensure((size_t)need);
+    p.atm_ent = r.ent.p;
+    p.atm_cap = need;
+    k_atm_list<true><<<gw, T, 0, s>>>(p);
+    return p;
+}
+
 // Diagnostics in the reference's apex convention: the lists and the ATM terms of the last
-// evaluation again, with the entries j <= a in caller order (the energies, forces and dE/dCN
-// summed over an atom's apex and entry shares are the same up to rounding).
-static void atm_reference_pass(Engine *e) {
-    if (!e->use_atm || !e->eval_current || (e->eval_opt.atm_surrogate && e->surr.loaded)) return;
+// evaluation again in the reference's order (the energies, forces and dE/dCN summed over an
+// atom's apex and entry shares are the same up to rounding). false: no evaluation that it can
+// repeat (none yet, another atom count set since, the surrogate)
+static bool atm_reference_pass(Engine *e, EvalLists &r) {
+    if (!e->use_atm || e->eval_n == 0 || e->eval_n != e->n || (e->eval_opt.atm_surrogate && e->surr.loaded)) return false;
     D3_CUDA(cudaDeviceSynchronize());
-    e->extra_visits = engine_extra_visits(e);
-    e->extra_known = true; // the lists are about to change their order
-    const Options now = e->opt;
-    e->opt = e->eval_opt;
+    EvalScope scope(e);
     const cudaStream_t s = e->stream;
     const size_t n = e->n;
-    for (int attempt = 0; attempt < 4; ++attempt) {
-        KP p = make_kp(e);
-        p.shard_rank = e->eval_rank;
-        p.shard_world = e->eval_world;
-        p.atm_ref_order = 1;
-        p.counters = nullptr;
-        double *sums[] = {p.ea, p.ga, p.fa, p.va, p.eb, p.gb, p.fb};
-        const int width[] = {1, 1, 3, 6, 1, 1, 3};
-        for (int k = 0; k < 7; ++k) D3_CUDA(cudaMemsetAsync(sums[k], 0, sizeof(double) * width[k] * n, s));
-        D3_CUDA(cudaMemsetAsync(e->gctl.p + 4, 0, 2 * sizeof(int), s));
-        launch_atm_lists(e, p, s);
-        if (e->nref == 5)
-            launch_atm_triplets<5>(e, p, s, false);
-        else
-            launch_atm_triplets<7>(e, p, s, false);
-        long long need = 0;
-        D3_CUDA(cudaMemcpyAsync(&need, e->atm_off.p + n, sizeof(long long), cudaMemcpyDeviceToHost, s));
-        D3_CUDA(cudaStreamSynchronize(s));
-        if (need <= e->atm_cap) break;
-        e->atm_cap = (long long)(need * 1.1) + 1024;
-        e->atm_ent.ensure((size_t)e->atm_cap);
+    KP p = eval_lists(e, r, true, s);
+    r.sums.ensure(16 * n);
+    D3_CUDA(cudaMemsetAsync(r.sums.p, 0, sizeof(double) * 16 * n, s));
+    double *q = r.sums.p;
+    double **const sums[] = {&p.ea, &p.ga, &p.fa, &p.va, &p.eb, &p.gb, &p.fb};
+    const int width[] = {1, 1, 3, 6, 1, 1, 3};
+    for (int k = 0; k < 7; ++k) {
+        *sums[k] = q;
+        q += width[k] * n;
     }
-    e->opt = now;
+    r.ea = p.ea;
+    r.ga = p.ga;
+    r.fa = p.fa;
+    r.va = p.va;
+    if (e->nref == 5)
+        launch_atm_triplets<5>(e, p, s, false);
+    else
+        launch_atm_triplets<7>(e, p, s, false);
+    D3_CUDA(cudaGetLastError());
+    D3_CUDA(cudaStreamSynchronize(s));
+    return true;
+}
+
+// additional visits of the last evaluation's triplets in the reference's enumeration: only
+// cells shorter than rc_ATM have any, and only asking for the counters pays for them
+static unsigned long long atm_repeated_visits(Engine *e) {
+    if (!e->use_atm || e->eval_n == 0 || (e->eval_opt.atm_surrogate && e->surr.loaded)) return 0;
+    bool images = false;
+    for (const SG &q : e->eval_geometry_moved ? e->eval_sg : e->sg)
+        images |= (q.atm_images[0] | q.atm_images[1] | q.atm_images[2]) != 0;
+    if (!images || (engine_fetch_status(e) & ST_LIST_OVERFLOW)) return 0; // (overflow: no ATM terms)
+    D3_CUDA(cudaDeviceSynchronize());
+    EvalScope scope(e);
+    const cudaStream_t s = e->stream;
+    EvalLists r;
+    const KP p = eval_lists(e, r, false, s);
+    r.repeats.ensure(1);
+    D3_CUDA(cudaMemsetAsync(r.repeats.p, 0, sizeof(unsigned long long), s));
+    k_atm_repeats<<<dim3(p.n, std::max(1, 4 * e->dev_sms / p.n)), REPEATS_THREADS, 0, s>>>(p, r.repeats.p);
+    D3_CUDA(cudaGetLastError());
+    unsigned long long six = 0;
+    D3_CUDA(cudaMemcpyAsync(&six, r.repeats.p, sizeof(six), cudaMemcpyDeviceToHost, s));
+    D3_CUDA(cudaStreamSynchronize(s));
+    return (six + 3) / 6; // (rounded: a distance equal to rc_ATM may be seen from one side only)
 }
 
 static void launch_group_reduce(const KP &p, int what, cudaStream_t s) {
@@ -2415,8 +2538,8 @@ static void launch_all(Engine *e, const KP &p0, cudaStream_t s, int stage = 0, d
         e->eval_rank = p.shard_rank;
         e->eval_world = p.shard_world;
         e->eval_opt = e->opt;
-        e->eval_current = true;
-        e->extra_known = false;
+        e->eval_n = e->n;
+        e->eval_geometry_moved = false;
         D3_CUDA(cudaEventRecord(ev[0], s));
         D3_CUDA(cudaMemsetAsync(p.counters, 0, sizeof(unsigned long long) * 4, s));
         D3_CUDA(cudaMemsetAsync(p.anyshift, 0, 7 * sizeof(int) * p.nstruct, s));
@@ -2543,7 +2666,7 @@ int engine_pass_times(Engine *e, float *ms, int cap, unsigned long long *counter
     for (; k < Engine::NEV - 1 && k < cap; ++k) D3_CUDA(cudaEventElapsedTime(&ms[k], e->ev[k], e->ev[k + 1]));
     if (counters) {
         D3_CUDA(cudaMemcpy(counters, e->counters.p, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost));
-        counters[0] += 2 * engine_extra_visits(e);
+        counters[0] += 2 * atm_repeated_visits(e);
     }
     return k;
 }
@@ -2731,7 +2854,8 @@ int engine_debug_pass_terms(Engine *e, double *out) {
     // virial[6]; chain-rule force[3], virial[6]; virials as xx yy zz xy xz yz, already
     // scaled by the pass's volume factor
     const uint64_t n = e->n;
-    atm_reference_pass(e);
+    EvalLists ref;
+    const bool again = atm_reference_pass(e, ref);
     std::vector<int> orig(n);
     D3_CUDA(cudaStreamSynchronize(e->stream));
     D3_CUDA(cudaMemcpy(orig.data(), e->orig.p, sizeof(int) * n, cudaMemcpyDeviceToHost));
@@ -2741,8 +2865,8 @@ int engine_debug_pass_terms(Engine *e, double *out) {
     };
     const bool atm = e->use_atm;
     const Col cols[] = {{e->e2.p, 1, 0}, {e->g2.p, 1, 1}, {e->f2.p, 3, 2}, {e->v2.p, 6, 5},
-                        {atm ? e->ea.p : nullptr, 1, 11}, {atm ? e->ga.p : nullptr, 1, 12},
-                        {atm ? e->fa.p : nullptr, 3, 13}, {atm ? e->va.p : nullptr, 6, 16},
+                        {again ? ref.ea : (atm ? e->ea.p : nullptr), 1, 11}, {again ? ref.ga : (atm ? e->ga.p : nullptr), 1, 12},
+                        {again ? ref.fa : (atm ? e->fa.p : nullptr), 3, 13}, {again ? ref.va : (atm ? e->va.p : nullptr), 6, 16},
                         {e->fc.p, 3, 22}, {e->vc.p, 6, 25}};
     constexpr int W = 31;
     std::vector<double> buf(6 * n);
@@ -2759,17 +2883,18 @@ int64_t engine_debug_atm_pairs(Engine *e, int64_t *outp, int64_t cap) {
     // returns (apex, j, Tref_x, Tref_y, Tref_z) rows in caller indices and reference shifts
     if (!e->use_atm) return 0;
     const uint64_t n = e->n;
-    atm_reference_pass(e);
+    EvalLists ref;
+    const bool again = atm_reference_pass(e, ref);
     std::vector<long long> off(n + 1);
     std::vector<int> orig(n);
     std::vector<int4> sh(n);
     D3_CUDA(cudaStreamSynchronize(e->stream));
-    D3_CUDA(cudaMemcpy(off.data(), e->atm_off.p, sizeof(long long) * (n + 1), cudaMemcpyDeviceToHost));
+    D3_CUDA(cudaMemcpy(off.data(), again ? ref.off.p : e->atm_off.p, sizeof(long long) * (n + 1), cudaMemcpyDeviceToHost));
     D3_CUDA(cudaMemcpy(orig.data(), e->orig.p, sizeof(int) * n, cudaMemcpyDeviceToHost));
     D3_CUDA(cudaMemcpy(sh.data(), e->shift.p, sizeof(int4) * n, cudaMemcpyDeviceToHost));
     const long long tot = off[n];
     std::vector<int2> ent((size_t)tot);
-    if (tot) D3_CUDA(cudaMemcpy(ent.data(), e->atm_ent.p, sizeof(int2) * tot, cudaMemcpyDeviceToHost));
+    if (tot) D3_CUDA(cudaMemcpy(ent.data(), again ? ref.ent.p : e->atm_ent.p, sizeof(int2) * tot, cudaMemcpyDeviceToHost));
     if (!outp) return tot;
     int64_t k = 0;
     for (uint64_t a = 0; a < n && k < cap; ++a)
