@@ -48,7 +48,7 @@
 // many types and the surrogate fallback.
 
 constexpr int ATM64_THREADS = 512;  // threads of all CTAs of an SM together
-constexpr int ATM64_ROWS = 4096;    // entries set up at once (longer lists: in parts)
+constexpr int ATM64_ENTRIES = 4096; // entries set up at once at most (longer lists: in parts)
 constexpr int ATM64_CHUNKS = 64;    // chunks of 32 partners in a tile at most
 constexpr int ATM64_SEG = 4;        // chunks tested together
 constexpr int ATM64_GROUP = 32;     // mixed chunks of a row queued at once (a multiple of ATM64_SEG)
@@ -88,13 +88,16 @@ struct __align__(16) Atm64Row {
     int j, t, k, pad;      // atom, type, entry number
     float f[4];            // rounded position
 };
-// scratch of one CTA: the entries, and the rows of its split by type with their C6 weights
+// a row x: its entry and C6 weights
+struct Atm64X {
+    Atm64Row e;
+    double w[MAX_NREF + 1], dw[MAX_NREF + 1];
+};
+// scratch of one CTA: the entries set up at once, then the rows of its split by type
 struct Atm64Scratch {
-    Atm64Row entries[ATM64_ROWS];
-    struct Row {
-        Atm64Row e;
-        double w[MAX_NREF + 1], dw[MAX_NREF + 1];
-    } rows[ATM64_ROWS];
+    unsigned char *p;
+    size_t stride; // bytes per CTA
+    int entries;
 };
 
 // position of an entry relative to the apex
@@ -292,7 +295,7 @@ __device__ __forceinline__ void atm64_visit(double vx, double vy, double vz, dou
 }
 
 template <int NR, int KIND>
-__global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch *scratch, int tile_bytes, int tile_max) {
+__global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch scratch, int tile_bytes, int tile_max) {
     extern __shared__ __align__(16) unsigned char sm64[];
     constexpr int RQ = atm64_rowq(NR);
     const int ne = p.ne, nw = blockDim.x >> 5;
@@ -317,8 +320,9 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch *
     }
     if (warp_uniform(p.atm_off[p.n] > p.atm_cap ? 1 : 0)) return; // list overflowed: the host grows it and re-runs
     for (int k = tid; k < ne * ne; k += blockDim.x) r0sq[k] = p.r0ab[k] * p.r0ab[k];
-    Atm64Row *entries = scratch[blockIdx.x].entries;
-    Atm64Scratch::Row *rows = scratch[blockIdx.x].rows;
+    const int ecap = scratch.entries;
+    Atm64Row *entries = reinterpret_cast<Atm64Row *>(scratch.p + blockIdx.x * scratch.stride);
+    Atm64X *rows = reinterpret_cast<Atm64X *>(entries + ecap);
     const double third = 1.0 / 3.0;
     const double rc = sqrt(p.ratm2), cinv = 16.0 / (2.0 * rc);
     // FP32 range test: |d3 - half| <= half in range, but near either end of [0, 2 half] the
@@ -364,10 +368,10 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch *
         float4 *sC = sF + tile + 32;                                  // [ATM64_CHUNKS][2]: box of each chunk, sphere radius
         double2 *sR = reinterpret_cast<double2 *>(sC + 2 * ATM64_CHUNKS); // [types][tile + 1][RQ]
         double acc = 0; // this lane's apex sum (lanes 0..10: energy, dE/dCN, force, virial)
-        for (int b0 = 0; b0 < m; b0 += ATM64_ROWS) {
+        for (int b0 = 0; b0 < m; b0 += ecap) {
             // set up the entries in Hilbert order (counting sort on a 16^3, 8^3 or 4^3 grid,
             // whose curves are prefixes of one another) and list this split's rows by type
-            const int bn = min(ATM64_ROWS, m - b0);
+            const int bn = min(ecap, m - b0);
             const int hs = bn >= 1024 ? 0 : (bn >= 128 ? 3 : 6), ncell = ATM64_CELLS >> hs;
             auto cell_of = [&](const int2 ent) {
                 const double3 v = atm64_pos(p, g, xa, ent, p.xs[ent.x]);
@@ -400,7 +404,7 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch *
             __syncthreads();
             for (int k = tid; k < bn; k += blockDim.x)
                 if (entries[k].k % S == split) {
-                    Atm64Scratch::Row *r = rows + atomicAdd(&tpos[entries[k].t], 1);
+                    Atm64X *r = rows + atomicAdd(&tpos[entries[k].t], 1);
                     r->e = entries[k];
 #pragma unroll
                     for (int b = 0; b < NR; ++b) {
@@ -419,7 +423,7 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch *
                     if (tid == 0) s_row = r0;
                     for (int k = tid; k < cnt; k += blockDim.x) {
                         int j, tj;
-                        if (m <= ATM64_ROWS) {
+                        if (m <= ecap) {
                             const Atm64Row *src = entries + p0 + k;
                             j = src->j;
                             tj = src->t;

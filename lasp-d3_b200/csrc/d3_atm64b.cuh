@@ -24,7 +24,7 @@
 // CTAs per SM), batch of 48 structures 106 -> 98 ms.
 
 constexpr int ATM64B_WARPS = 12;   // warps per SM at most (168 registers a thread)
-constexpr int ATM64B_MCAP = 4096;  // longest list (longer ones: k_atm64)
+constexpr int ATM64B_MCAP = 4096;  // longest list at most (KP::atmb_mcap; longer ones: k_atm64)
 constexpr int ATM64B_NACC = 8;     // accumulators per entry: E, dE/dCN, force, virial coefficient
 constexpr int ATM64B_STATIC = 2560;
 
@@ -37,13 +37,11 @@ __host__ __device__ inline size_t atm64b_fixed(int ne, int NR) {
 __host__ __device__ inline size_t atm64b_warp(int ne, int NR, bool simple) {
     return 32 * ((size_t)ne * atm64b_row(NR) * sizeof(double) + 3 * sizeof(double2) + sizeof(float4) + (simple ? 0 : 6 * sizeof(double)));
 }
-struct Atm64bScratch {
-    Atm64Row entries[ATM64B_MCAP];
-    double acc[ATM64B_MCAP][ATM64B_NACC];
-};
+// scratch of one CTA: atmb_mcap entries, then their accumulators
+constexpr size_t ATM64B_ENTRY_BYTES = sizeof(Atm64Row) + ATM64B_NACC * sizeof(double);
 
 template <int NR, bool SIMPLE>
-__global__ void __launch_bounds__(ATM64B_WARPS * 32, 1) k_atm64b(KP p, Atm64bScratch *scratch) {
+__global__ void __launch_bounds__(ATM64B_WARPS * 32, 1) k_atm64b(KP p, unsigned char *scratch) {
     extern __shared__ __align__(16) unsigned char sm64b[];
     constexpr int RW = atm64b_row(NR) / 2; // double2 words per row
     const int ne = p.ne, nw = blockDim.x >> 5;
@@ -62,8 +60,8 @@ __global__ void __launch_bounds__(ATM64B_WARPS * 32, 1) k_atm64b(KP p, Atm64bScr
     __shared__ double red[ATM64B_WARPS][12];
     if (warp_uniform(p.atm_off[p.n] > p.atm_cap ? 1 : 0)) return; // list overflowed: the host grows it and re-runs
     for (int k = tid; k < ne * ne; k += blockDim.x) r0sq[k] = p.r0ab[k] * p.r0ab[k];
-    Atm64Row *entries = scratch[blockIdx.x].entries;
-    double (*acc)[ATM64B_NACC] = scratch[blockIdx.x].acc;
+    Atm64Row *entries = reinterpret_cast<Atm64Row *>(scratch + blockIdx.x * (ATM64B_ENTRY_BYTES * p.atmb_mcap));
+    double (*acc)[ATM64B_NACC] = reinterpret_cast<double (*)[ATM64B_NACC]>(entries + p.atmb_mcap);
     const double rc = sqrt(p.ratm2), cinv = 16.0 / (2.0 * rc);
     const float half = (float)(0.5 * p.ratm2 * (1.0 + 1e-5)), sure = half * (1.0f - 4e-5f);
     const float rc_hi = (float)(p.ratm2 * (1.0 + 1e-4));
@@ -79,7 +77,7 @@ __global__ void __launch_bounds__(ATM64B_WARPS * 32, 1) k_atm64b(KP p, Atm64bScr
         const SG &g = p.sg[p.sid[a]];
         const long long e0 = p.atm_off[a];
         const int m = warp_uniform((int)(p.atm_off[a + 1] - e0));
-        if (m > ATM64B_MCAP || warp_uniform(g.atm_simple) != (SIMPLE ? 1 : 0)) continue; // k_atm64's, the other instance's
+        if (m > p.atmb_mcap || warp_uniform(g.atm_simple) != (SIMPLE ? 1 : 0)) continue; // k_atm64's, the other instance's
         const bool ref = !SIMPLE && atm_reference_order(p, g, p.sid[a]);
         const double4 xa = p.xs[a];
         for (int k = tid; k < ne * NR; k += blockDim.x) yapex[k] = p.Y[(size_t)a * ne * NR + k];

@@ -68,7 +68,6 @@ struct SG {
     int stcb_off, stcb_n;     // CN / chain-rule stencil of the same blocks
     int stab_off, stab_n;     // rc_ATM stencil of the same blocks (ATM half lists)
     int atm_simple;           // every cell height > 2 rc_ATM: no atom twice in an ATM list
-    int atm_images[3];        // lattice vectors within rc_ATM span at most +- this many cells
     double ratm_frac[3];      // rc_ATM over the cell heights
 };
 
@@ -132,7 +131,7 @@ struct KP {
                     // the type pair, the row of the weight derivatives, the atom index bits
     double *YD64;   // [n][ne][atm64b_row]: the same rows in FP64: Y, D, r0^2
     int atm_min_m;  // k_atm32 / k_atm64 take only apexes with longer lists (the rest: block pairs)
-    int atmb_mcap;  // longest list k_atm32b takes
+    int atmb_mcap;  // longest list the block pairs (k_atm32b, k_atm64b) take
     int atmb_split; // CTAs of k_atm32b sharing one apex (each a share of its block rows)
     // sharded evaluation: this process computes the two-body and chain-rule terms of the
     // atom groups it owns (group_owner; without groups: central atoms i = shard_rank +
@@ -1227,6 +1226,46 @@ struct DBuf {
     }
 };
 
+// work space whose size follows the structures: a captured graph keeps the address it was
+// captured with, so a buffer that became too small stays until the handle goes (growing by
+// at least half, all of them together take less than three times the last)
+struct KeptBuf {
+    unsigned char *p = nullptr;
+    size_t n = 0;
+    std::vector<unsigned char *> old;
+    void ensure(size_t m) {
+        if (m <= n) return;
+        unsigned char *q = nullptr;
+        const size_t want = std::max(m, n + n / 2);
+        D3_CUDA(cudaMalloc(&q, want));
+        if (p) old.push_back(p);
+        p = q;
+        n = want;
+    }
+    void release() {
+        for (unsigned char *q : old) cudaFree(q);
+        old.clear();
+        if (p) cudaFree(p);
+        p = nullptr;
+        n = 0;
+    }
+};
+
+// FP64 ATM pass of one evaluation
+struct Atm64bShape {
+    int warps, ctas; // per CTA, per SM
+};
+struct Atm64Plan {
+    // block pairs (weight-free structures, the others): none where a kind present has no shape
+    bool blocks = false;
+    Atm64bShape block[2] = {{0, 1}, {0, 1}};
+    int block_split[2] = {1, 1}, block_grid[2] = {0, 0}, block_cap = 0; // entries of the longest list
+    // rows: CTAs per SM, splits of an apex, shared memory, entries set up at once
+    int ctas = 1, split = 1, grid = 0, entries = 0;
+    size_t fixed = 0, tile_bytes = 0, stride = 0;
+    unsigned char *scratch = nullptr;
+};
+
 // learned ATM surrogate: model on the device and its per-evaluation work arrays
 struct SurrState {
     bool loaded = false;
@@ -1292,8 +1331,8 @@ struct Engine {
     DBuf<float4> xs32;
     DBuf<float> w32, dw32, Y32, YD32;
     DBuf<float4> atmb_scratch;
-    DBuf<Atm64Scratch> atm64_scratch;
-    DBuf<Atm64bScratch> atm64b_scratch;
+    KeptBuf atm64_scratch; // k_atm64b and, behind it, k_atm64
+    Atm64Plan atm64;       // of the evaluation at hand
     DBuf<double> YD64;
     DBuf<long long> atm_off;
     DBuf<int2> atm_ent;
@@ -1348,7 +1387,6 @@ struct Engine {
         YD32.release();
         atmb_scratch.release();
         atm64_scratch.release();
-        atm64b_scratch.release();
         YD64.release();
         xw_in.release();
         xs.release();
@@ -1653,10 +1691,7 @@ static void build_structures(Engine *e, int nstruct, const uint64_t *counts, con
         // a nonzero lattice vector is at least as long as the smallest height, so with every
         // height above 2 rc_ATM two images of one atom never lie within rc_ATM of an apex
         r.atm_simple = std::min(g.height[0], std::min(g.height[1], g.height[2])) > 2.0 * e->rc_atm * (1.0 + 1e-9);
-        for (int i = 0; i < 3; ++i) {
-            r.ratm_frac[i] = e->use_atm ? e->rc_atm / g.height[i] : 0.0;
-            r.atm_images[i] = (int)std::min(std::floor(r.ratm_frac[i] * (1.0 + 1e-9)), 1024.0);
-        }
+        for (int i = 0; i < 3; ++i) r.ratm_frac[i] = e->use_atm ? e->rc_atm / g.height[i] : 0.0;
         int64_t mcb[3];
         r.box_mode = reference_box(cells_f + 9 * k, e->rc_f, e->rc_cn_f, mcb) ? 1 : 0;
         for (int i = 0; i < 3; ++i) r.half[i] = (int)(mcb[i] / 2);
@@ -1959,9 +1994,6 @@ static int apex_split(long long apexes, long long ctas, int most, double setup) 
 // visits of another (8,000 atoms 157 -> 154 ms, 4,000 atoms of short lists 2.93 -> 2.50 ms);
 // one for the others, whose virial carries leave room for fewer warps in halves (2,000 atoms
 // 44.2 against 46.2 ms, batch of 48 structures 98 against 108 ms).
-struct Atm64bShape {
-    int warps, ctas; // per CTA, per SM
-};
 static Atm64bShape atm64b_shape(const Engine *e, bool simple) {
     if (!e->use_atm || e->opt.precision || e->opt.atm_schedule != 0 || (e->opt.atm_surrogate && e->surr.loaded)) return {0, 1};
     if (4 * e->n < (uint64_t)e->dev_sms) return {0, 1};
@@ -1979,27 +2011,91 @@ static Atm64bShape atm64b_shape(const Engine *e, bool simple) {
     return {0, 1};
 }
 
-// CTAs per SM of the FP64 ATM kernel, their shared memory and the splits of an apex
-struct Atm64Shape {
-    int ctas, split;
-    size_t fixed, tile_bytes;
-};
-static Atm64Shape atm64_shape(const Engine *e, int world) {
-    Atm64Shape sh;
-    const int want = e->opt.atm_ctas_per_sm;
-    sh.ctas = want <= 0 ? 1 : (want >= 4 ? 4 : (want >= 2 ? 2 : 1));
-    const size_t limit = std::min<size_t>(227 * 1024, 228 * 1024 / sh.ctas - 1024) - ATM64_STATIC;
-    sh.fixed = atm64_fixed_bytes(e->ne, e->nref, ATM64_THREADS / 32 / sh.ctas);
-    sh.tile_bytes = limit - sh.fixed;
-    sh.split = apex_split(std::max<long long>(1, (long long)e->n / std::max(1, world)), e->dev_sms * sh.ctas, 32, 0.01);
-    return sh;
+// Entries that a CTA of the FP64 ATM kernels has room for: twice the mean half list of the
+// densest structure (slabs and clusters in vacuum; centre mode: full lists) and some, at most
+// what the images within rc_ATM allow. Longer lists are right too, k_atm64 takes them in parts.
+static int atm64_entries(const Engine *e, bool center) {
+    double most = 0.0;
+    for (size_t k = 0; k < e->sg.size(); ++k) {
+        const SG &q = e->sg[k];
+        const double mean = (center ? 1.0 : 0.5) * 4.18879020478639 * e->rc_atm * e->rc_atm * e->rc_atm * q.natoms / std::fabs(e->geoms[k].volume);
+        double images = q.natoms;
+        for (int i = 0; i < 3; ++i) images *= std::floor(2.0 * q.ratm_frac[i]) + 1.0;
+        most = std::max(most, std::min(images, std::max(1024.0, 2.0 * mean + 256.0)));
+    }
+    return (int)(std::ceil(std::min(most, (double)ATM64_ENTRIES) / 256.0) * 256.0);
 }
 
-static KP make_kp(Engine *e) {
+static size_t atm64_stride(int entries, int split) {
+    return (size_t)entries * sizeof(Atm64Row) + (size_t)((entries + split - 1) / split) * sizeof(Atm64X);
+}
+
+// The FP64 ATM pass over an evaluation's structures. Its scratch, for the CTAs that have an
+// item, is what the block pairs need or, without them, the rows: with lists of 2,000 entries
+// 71 MB for 16 atoms and 97 MB from 37 on (194 MB weight-free; room for 4,096 rows in every
+// CTA beside that was another 194 MB for any handle). Nothing is allocated while the stream is being captured: block pairs then
+// take shorter lists, or none, and the rows are set up in shorter parts (in the FP32 form's
+// scratch, if the evaluations before were of that form).
+static Atm64Plan atm64_plan(Engine *e, cudaStream_t s, int world) {
+    Atm64Plan q;
+    const bool center = e->opt.atm_surrogate && e->surr.loaded;
+    const long long apexes = std::max<long long>(1, ((long long)e->n + world - 1) / world);
+    const int want = e->opt.atm_ctas_per_sm;
+    q.ctas = want <= 0 ? 1 : (want >= 4 ? 4 : (want >= 2 ? 2 : 1));
+    const size_t limit = std::min<size_t>(227 * 1024, 228 * 1024 / q.ctas - 1024) - ATM64_STATIC;
+    q.fixed = atm64_fixed_bytes(e->ne, e->nref, ATM64_THREADS / 32 / q.ctas);
+    q.tile_bytes = limit - q.fixed;
+    q.split = center ? 1 : apex_split(std::max<long long>(1, (long long)e->n / world), e->dev_sms * q.ctas, 32, 0.01);
+    q.grid = (int)std::min<long long>((long long)e->dev_sms * q.ctas, apexes * q.split);
+    q.entries = atm64_entries(e, center);
+    bool kind[2] = {false, false};
+    for (const SG &g : e->sg) kind[g.atm_simple ? 0 : 1] = true;
+    q.blocks = !center;
+    int widest = 0;
+    for (int k = 0; k < 2; ++k) {
+        if (!kind[k]) continue;
+        q.block[k] = atm64b_shape(e, k == 0);
+        q.blocks = q.blocks && q.block[k].warps > 0;
+        const int grid = e->dev_sms * q.block[k].ctas;
+        q.block_split[k] = apex_split(std::max<long long>(1, (long long)e->n / world), grid, 32, 0.02);
+        q.block_grid[k] = (int)std::min<long long>(grid, apexes * q.block_split[k]);
+        widest = std::max(widest, q.block_grid[k]);
+    }
+    q.block_cap = std::min(q.entries, ATM64B_MCAP);
+    const size_t yd = (size_t)e->max_atoms * e->ne * atm64b_row(e->nref);
+    size_t have = e->atm64_scratch.n;
+    q.scratch = e->atm64_scratch.p;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
+    const bool grow = capture == cudaStreamCaptureStatusNone;
+    if (!grow && have == 0) {
+        q.scratch = reinterpret_cast<unsigned char *>(e->atmb_scratch.p);
+        have = e->atmb_scratch.n * sizeof(*e->atmb_scratch.p);
+    }
+    if (q.blocks && grow) {
+        e->YD64.ensure(yd);
+        e->atm64_scratch.ensure(widest * ATM64B_ENTRY_BYTES * q.block_cap);
+    } else if (q.blocks) {
+        q.block_cap = (int)std::min<size_t>(q.block_cap, have / widest / ATM64B_ENTRY_BYTES / 32 * 32);
+        q.blocks = e->YD64.n >= yd && q.block_cap >= 256;
+    }
+    // behind block pairs the rows make do with their scratch: only lists too long for those
+    if (q.blocks && grow) have = widest * ATM64B_ENTRY_BYTES * q.block_cap;
+    const bool fit = q.blocks || !grow;
+    while (fit && q.entries > 32 && q.grid * atm64_stride(q.entries, q.split) > have) q.entries -= 32;
+    q.stride = atm64_stride(q.entries, q.split);
+    if (grow || q.grid * q.stride > have) {
+        e->atm64_scratch.ensure(q.grid * q.stride);
+        q.scratch = e->atm64_scratch.p;
+    }
+    return q;
+}
+
+static KP make_kp(Engine *e, cudaStream_t s, int rank = 0, int world = 1) {
     KP p;
     memset(&p, 0, sizeof(p));
-    p.shard_rank = 0;
-    p.shard_world = 1;
+    p.shard_rank = rank;
+    p.shard_world = world;
     p.n = (int)e->n;
     p.nstruct = e->nstruct;
     p.nbins_total = e->nbins_total;
@@ -2052,17 +2148,9 @@ static KP make_kp(Engine *e) {
                                              : apex_split(std::max(1, p.n), ctas, 16, 0.05);
     }
     p.YD64 = nullptr;
-    const Atm64bShape shb[2] = {atm64b_shape(e, true), atm64b_shape(e, false)};
-    if (shb[0].warps > 0 || shb[1].warps > 0) {
-        bool simple = false;
-        for (const SG &q : e->sg) simple |= q.atm_simple != 0;
-        e->YD64.ensure((size_t)e->max_atoms * e->ne * atm64b_row(e->nref));
-        e->atm64b_scratch.ensure((size_t)e->dev_sms * (simple ? shb[0].ctas : 1));
-        p.YD64 = e->YD64.p;
-    }
     if (e->use_atm && !p.precision) {
-        const Atm64Shape sh = atm64_shape(e, 1);
-        e->atm64_scratch.ensure((size_t)e->dev_sms * sh.ctas);
+        e->atm64 = atm64_plan(e, s, world);
+        if (e->atm64.blocks) p.YD64 = e->YD64.p;
     }
     p.atm_force_scaled = e->opt.atm_force_scaled ? 1 : 0;
     p.anyshift = e->anyshift.p;
@@ -2174,42 +2262,40 @@ static void launch_blockpair(Engine *e, const KP &p, cudaStream_t s, const AtmbS
 template <int NR>
 static void launch_atm64(Engine *e, const KP &p0, cudaStream_t s, bool center) {
     KP p = p0;
-    const Atm64Shape sh = atm64_shape(e, p.shard_world);
-    p.atmb_split = sh.split;
-    const size_t sm = sh.fixed + sh.tile_bytes;
-    const int tile_max = e->opt.atm_tile > 0 ? std::max(32, std::min(e->opt.atm_tile, 65504) & ~31) : 65504;
-    const int grid = e->dev_sms * sh.ctas;
+    const Atm64Plan &q = e->atm64;
     bool kind[3] = {false, false, center};
     if (!center)
-        for (const SG &q : e->sg) kind[q.atm_simple ? ATM64_SIMPLE : ATM64_WEIGHTED] = true;
+        for (const SG &g : e->sg) kind[g.atm_simple ? ATM64_SIMPLE : ATM64_WEIGHTED] = true;
+    if (q.blocks) {
+        // lists up to block_cap entries; longer ones below
+        const void *fnb[2] = {(const void *)k_atm64b<NR, true>, (const void *)k_atm64b<NR, false>};
+        p.atmb_mcap = q.block_cap;
+        for (int k = 0; k < 2; ++k) {
+            if (!kind[k]) continue;
+            p.atmb_split = q.block_split[k];
+            const size_t smb = atm64b_fixed(p.ne, NR) + q.block[k].warps * atm64b_warp(p.ne, NR, k == ATM64_SIMPLE);
+            if (k == 1 && kind[0]) D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
+            atm_occupancy(e, 6 + k, smb, fnb[k]);
+            void *args[] = {(void *)&p, (void *)&q.scratch};
+            D3_CUDA(cudaLaunchKernel(fnb[k], dim3(q.block_grid[k]), dim3(32 * q.block[k].warps), args, smb, s));
+        }
+        D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
+        p.atm_min_m = q.block_cap;
+    }
     const void *fns[3] = {(const void *)k_atm64<NR, ATM64_SIMPLE>, (const void *)k_atm64<NR, ATM64_WEIGHTED>,
                           (const void *)k_atm64<NR, ATM64_CENTER>};
     const int cache[3] = {0, 4, 2};
-    const Atm64bShape shapes[2] = {atm64b_shape(e, true), atm64b_shape(e, false)}; // ATM64_SIMPLE, ATM64_WEIGHTED
-    if (!center && (!kind[0] || shapes[0].warps > 0) && (!kind[1] || shapes[1].warps > 0)) {
-        // lists up to ATM64B_MCAP entries: block pairs; longer ones below
-        KP q = p;
-        const void *fnb[2] = {(const void *)k_atm64b<NR, true>, (const void *)k_atm64b<NR, false>};
-        for (int k = 0; k < 2; ++k) {
-            if (!kind[k]) continue;
-            const int nw = shapes[k].warps, grid_b = e->dev_sms * shapes[k].ctas;
-            q.atmb_split = apex_split(std::max(1, p.n / p.shard_world), grid_b, 32, 0.02);
-            const size_t smb = atm64b_fixed(p.ne, NR) + nw * atm64b_warp(p.ne, NR, k == ATM64_SIMPLE);
-            if (k == 1 && kind[0]) D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
-            atm_occupancy(e, 6 + k, smb, fnb[k]);
-            void *args[] = {(void *)&q, (void *)&e->atm64b_scratch.p};
-            D3_CUDA(cudaLaunchKernel(fnb[k], dim3(grid_b), dim3(32 * nw), args, smb, s));
-        }
-        D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
-        p.atm_min_m = ATM64B_MCAP;
-    }
+    const size_t sm = q.fixed + q.tile_bytes;
+    int tile_bytes = (int)q.tile_bytes;
+    int tile_max = e->opt.atm_tile > 0 ? std::max(32, std::min(e->opt.atm_tile, 65504) & ~31) : 65504;
+    Atm64Scratch scratch{q.scratch, q.stride, q.entries};
+    p.atmb_split = q.split;
     for (int k = 0; k < 3; ++k) {
         if (!kind[k]) continue;
         if (k == ATM64_WEIGHTED && kind[ATM64_SIMPLE]) D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
         atm_occupancy(e, cache[k], sm, fns[k]);
-        int tile_bytes = (int)sh.tile_bytes, tmax = tile_max;
-        void *args[] = {(void *)&p, (void *)&e->atm64_scratch.p, &tile_bytes, &tmax};
-        D3_CUDA(cudaLaunchKernel(fns[k], dim3(grid), dim3(ATM64_THREADS / sh.ctas), args, sm, s));
+        void *args[] = {(void *)&p, (void *)&scratch, &tile_bytes, &tile_max};
+        D3_CUDA(cudaLaunchKernel(fns[k], dim3(q.grid), dim3(ATM64_THREADS / q.ctas), args, sm, s));
     }
 }
 
@@ -2253,7 +2339,9 @@ __global__ void __launch_bounds__(REPEATS_THREADS) k_atm_repeats(KP p, unsigned 
     const int a = blockIdx.x, sid = p.sid[a];
     const SG &g = p.sg[sid];
     if (atm_reference_order(p, g, sid)) return;
-    const int kx = g.atm_images[0], ky = g.atm_images[1], kz = g.atm_images[2];
+    // lattice vectors within rc_ATM span at most +- this many cells
+    auto reach = [&](int k) { return (int)fmin(floor(g.ratm_frac[k] * (1.0 + 1e-9)), 1024.0); };
+    const int kx = reach(0), ky = reach(1), kz = reach(2);
     const int wx = 2 * kx + 1, wy = 2 * ky + 1;
     const long long box = (long long)wx * wy * (2 * kz + 1);
     if (box == 1) return;
@@ -2427,9 +2515,7 @@ static KP eval_lists(Engine *e, EvalLists &r, bool ref_order, cudaStream_t s) {
     D3_CUDA(cudaMemcpyAsync(r.sg.p, e->sg.data(), sizeof(SG) * e->sg.size(), cudaMemcpyHostToDevice, s));
     D3_CUDA(cudaMemcpyAsync(r.rows.p, e->stencil_rows.data(), sizeof(int4) * e->stencil_rows.size(), cudaMemcpyHostToDevice, s));
     D3_CUDA(cudaMemsetAsync(r.bins.p, 0, sizeof(int) * nbins, s));
-    KP p = make_kp(e);
-    p.shard_rank = e->eval_rank;
-    p.shard_world = e->eval_world;
+    KP p = make_kp(e, s, e->eval_rank, e->eval_world);
     p.atm_ref_order = ref_order ? 1 : 0;
     p.counters = nullptr;
     p.nstruct = (int)e->sg.size();
@@ -2496,7 +2582,7 @@ static unsigned long long atm_repeated_visits(Engine *e) {
     if (!e->use_atm || e->eval_n == 0 || (e->eval_opt.atm_surrogate && e->surr.loaded)) return 0;
     bool images = false;
     for (const SG &q : e->eval_geometry_moved ? e->eval_sg : e->sg)
-        images |= (q.atm_images[0] | q.atm_images[1] | q.atm_images[2]) != 0;
+        images |= std::max(q.ratm_frac[0], std::max(q.ratm_frac[1], q.ratm_frac[2])) * (1.0 + 1e-9) >= 1.0;
     if (!images || (engine_fetch_status(e) & ST_LIST_OVERFLOW)) return 0; // (overflow: no ATM terms)
     D3_CUDA(cudaDeviceSynchronize());
     EvalScope scope(e);
@@ -2795,7 +2881,7 @@ uint16_t engine_compute(Engine *e, double *energy, double *forces, double *stres
         ensure_atm_capacity(e);
         for (int attempt = 0; attempt < 4; ++attempt) {
             D3_CUDA(cudaMemsetAsync(e->status.p, 0, sizeof(unsigned int), s));
-            KP p = make_kp(e);
+            KP p = make_kp(e, s);
             if (e->nref == 5)
                 launch_all<5>(e, p, s);
             else
@@ -3028,7 +3114,7 @@ int engine_surrogate_descriptors(Engine *e, const int *channel_z, int nch, float
         S.xcenter.ensure(std::max<size_t>(n, 1));
         D3_CUDA(cudaMemcpy(S.xchan.p, chan.data(), sizeof(int) * e->ne, cudaMemcpyHostToDevice));
         if (n == 0) return 0;
-        KP p = make_kp(e);
+        KP p = make_kp(e, s);
         const SurrDesc sd = surr_desc(S.xchan.p, nch, S.xG.p, nullptr, S.xcenter.p);
         const int T = 256;
         const int gw = (int)(((long long)n * 32 + T - 1) / T);
@@ -3064,9 +3150,7 @@ uint16_t engine_shard_begin(Engine *e, int rank, int world, double *G_out, cudaS
         ensure_atm_capacity(e);
         for (int attempt = 0; attempt < 4; ++attempt) {
             D3_CUDA(cudaMemsetAsync(e->status.p, 0, sizeof(unsigned int), s));
-            KP p = make_kp(e);
-            p.shard_rank = rank;
-            p.shard_world = world;
+            KP p = make_kp(e, s, rank, world);
             if (e->nref == 5)
                 launch_all<5>(e, p, s, 1, G_out);
             else
@@ -3099,9 +3183,7 @@ uint16_t engine_shard_end(Engine *e, const double *G_in, double *out_dev, cudaSt
     }
     cudaStream_t s = stream ? stream : e->stream;
     try {
-        KP p = make_kp(e);
-        p.shard_rank = e->shard_rank;
-        p.shard_world = e->shard_world;
+        KP p = make_kp(e, s, e->shard_rank, e->shard_world);
         if (e->nref == 5)
             launch_all<5>(e, p, s, 2, const_cast<double *>(G_in));
         else
