@@ -6,17 +6,19 @@ Tunables (engine options):
                             one lane each) or 32 (one warp per atom)
   D3_OPT_ATMB_WARPS         block-pair ATM kernel: warps per CTA (up to 8 with (ATM pass,
                             two y buffers per warp, 9-12 with one)               precision)
-  D3_OPT_ATM_CTAS_PER_SM    CTAs per SM (block-pair: 2 CTAs of 4 warps when they fit;
-                            mirror / FP64 kernels: persistent CTAs per SM)
+  D3_OPT_ATM_CTAS_PER_SM    CTAs per SM (precision block pairs: 2 CTAs of 4 warps when they
+                            fit; FP64 row kernel and mirror kernel: persistent CTAs per SM)
   D3_OPT_ATMB_LIST_CAPACITY longest list of the block-pair kernel (the rest go to the
                             mirror kernel)
   D3_OPT_ATMB_FINE_SKIP     block-pair kernel: skip out-of-range visits per two steps
-  D3_OPT_ATM_TILE           partner-tile entries of the mirror and FP64 ATM kernels
+  D3_OPT_ATM_TILE           partner-tile entries of the FP64 row kernel and the mirror kernel
 
 `tune(handle, key)` times each candidate with the engine's per-pass CUDA-event timers
 (d3_pass_times) on the caller's own workload and keeps the fastest; the pair passes and
 the ATM pass are tuned independently (bin width and pair kernel first, then the ATM
-kernel's shape: block-pair shapes in the precision form, tile and CTAs in the FP64 form).
+kernel's shape: block-pair shapes in the precision form, tile and CTAs in the FP64 form
+where its row kernel takes the lists; its block pairs have nothing to tune, and what they
+leave to the row kernel runs at the defaults).
 Results are cached in a JSON file keyed by GPU name, atom-count bucket (powers of two),
 density bucket, cutoffs, ATM on/off and precision form, so a workload of the same kind
 reuses them without timing. Cache path: $D3_AUTOTUNE_CACHE or
@@ -26,12 +28,13 @@ import json
 import math
 import os
 
-from d3_b200 import (OPT_ATM_CTAS_PER_SM, OPT_ATM_TILE, OPT_ATMB_FINE_SKIP, OPT_ATMB_LIST_CAPACITY, OPT_ATMB_WARPS,
-                     OPT_BIN_DIVISOR, OPT_PAIR_KERNEL)
+from d3_b200 import (OPT_ATM_CTAS_PER_SM, OPT_ATM_SCHEDULE, OPT_ATM_TILE, OPT_ATMB_FINE_SKIP, OPT_ATMB_LIST_CAPACITY,
+                     OPT_ATMB_WARPS, OPT_BIN_DIVISOR, OPT_PAIR_KERNEL)
 
 BIN_DIVISORS = (3, 4, 6, 8)
 PAIR_KERNELS = (0, 1)
-ATM_TILES = (64, 128, 256)
+# FP64 row kernel; 0, its default, is all partners of an apex (up to 2,048) in one CTA per SM
+ATM_TILES = (0, 128, 256)
 ATM_CTAS = (0, 2, 3)
 # block-pair shapes: (warps per CTA, CTAs per SM, list capacity; 0 = automatic; skip
 # out-of-range visits per two steps)
@@ -56,8 +59,8 @@ def workload_key(n_atoms, volume_a3, rc, rc_cn, rc_atm, precision):
     nb = int(round(math.log2(max(n_atoms, 1))))
     rho = n_atoms / max(volume_a3, 1e-9)
     rb = round(math.log2(rho) * 2) / 2 if rho > 0 else 0
-    # v2: the parameter set includes the pair kernel and the block-pair ATM shape
-    return "v2|%s|n2^%d|rho2^%.1f|rc%.1f/%.1f/%.1f|p%d" % (gpu_name(), nb, rb, rc, rc_cn, rc_atm or 0.0, precision)
+    # v3: FP64 tiles and CTAs of the row kernel (v2's were measured for another kernel)
+    return "v3|%s|n2^%d|rho2^%.1f|rc%.1f/%.1f/%.1f|p%d" % (gpu_name(), nb, rb, rc, rc_cn, rc_atm or 0.0, precision)
 
 
 def _load():
@@ -92,6 +95,17 @@ def _time(handle, repeats):
         pt, _ = handle.pass_times()
         best = pt if best is None else {k: min(best[k], pt[k]) for k in pt}
     return best
+
+
+def _by_rows(handle):
+    """Whether the FP64 row kernel takes the ATM pass (block pairs are one launch more)."""
+    if not hasattr(handle, "launches_per_eval") or handle.options.get(OPT_ATM_SCHEDULE, 0) != 0:
+        return True
+    launches = handle.launches_per_eval()
+    handle.set_option(OPT_ATM_SCHEDULE, 1)
+    rows = handle.launches_per_eval()
+    handle.set_option(OPT_ATM_SCHEDULE, 0)
+    return launches == rows
 
 
 def tune(handle, key, repeats=2, use_cache=True, atm=True, precision=None):
@@ -137,7 +151,7 @@ def tune(handle, key, repeats=2, use_cache=True, atm=True, precision=None):
                     best = (t, w, c, m, f)
             (params["atmb_warps"], params["atm_ctas_per_sm"], params["atmb_mcap"],
              params["atmb_fine_skip"]) = best[1:]
-        else:
+        elif _by_rows(handle):
             for tile in ATM_TILES:
                 for ctas in ATM_CTAS:
                     handle.set_option(OPT_ATM_TILE, tile)

@@ -242,10 +242,12 @@ class D3(_Surrogate, _Shard):
         if not self.h:
             raise RuntimeError("d3_init_handle_ex failed: %s" % self.lib.d3_last_error().decode())
         self.n = 0
+        self.options = {}  # as set through set_option
 
     def set_option(self, opt, value):
         if self.lib.d3_set_option(self.h, int(opt), int(value)):
             raise RuntimeError(self.lib.d3_last_error().decode())
+        self.options[int(opt)] = int(value)
 
     def set_functional_params(self, s6, s8, p1, p2):
         self.lib.d3_set_functional_params(self.h, s6, s8, p1, p2)
@@ -368,10 +370,12 @@ class D3Batch(_Surrogate, _Shard):
         if not self.h:
             raise RuntimeError("d3_init_batch failed: %s" % self.lib.d3_last_error().decode())
         self.counts = None
+        self.options = {}  # as set through set_option
 
     def set_option(self, opt, value):
         if self.lib.d3_set_option(self.h, int(opt), int(value)):
             raise RuntimeError(self.lib.d3_last_error().decode())
+        self.options[int(opt)] = int(value)
 
     def set_structures(self, structures):
         """structures: list of dicts with pos [n,3], Z [n], cell [3,3] (Angstrom)."""
