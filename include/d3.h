@@ -114,8 +114,12 @@ enum {
                                     triplet arithmetic with FP64 C6 weights, dE/dCN and final
                                     reductions (precision form) */
     D3_OPT_BIN_DIVISOR = 4,      /* cell-list bin width = smallest cutoff / value (1..32, default 6) */
-    D3_OPT_ATM_TILE = 5,         /* ATM partner tile entries (0 = automatic) */
-    D3_OPT_ATM_CTAS_PER_SM = 6,  /* persistent ATM CTAs per SM (0 = occupancy limit) */
+    D3_OPT_ATM_TILE = 5,         /* ATM partner tile entries (0 = automatic: as many as fit, 128
+                                    in the precision form); not for block pairs */
+    D3_OPT_ATM_CTAS_PER_SM = 6,  /* persistent ATM CTAs per SM. FP64: 1..8, as many as fit (0 =
+                                    one); its block pairs choose their own. Precision form:
+                                    up to the occupancy limit (0 = that limit), block pairs
+                                    see D3_OPT_ATMB_WARPS */
     D3_OPT_ATM_SCHEDULE = 8,     /* ATM: 0 (default) block pairs, each triplet visited once
                                     (FP64: where apexes and lists are large enough for it);
                                     1 mirror-symmetric, each triplet twice */
@@ -132,16 +136,17 @@ enum {
                                     automatic (8), 2..12; above 8 each warp stages one y
                                     block at a time instead of two. With
                                     D3_OPT_ATM_CTAS_PER_SM = 2, two CTAs per SM when they fit */
-    D3_OPT_ATMB_LIST_CAPACITY = 12, /* longest half list (entries) the block-pair kernel takes,
-                                    0 = as many as the shared memory allows (4,096..8,192);
+    D3_OPT_ATMB_LIST_CAPACITY = 12, /* longest half list (entries) the precision form's
+                                    block-pair kernel takes, 0 = as many as the shared memory allows (4,096..8,192);
                                     longer lists go to the mirror-symmetric kernel */
-    D3_OPT_ATMB_SPLIT = 13,      /* CTAs of the block-pair kernel sharing one apex, each taking
-                                    every S-th block row (0 = automatic: the S that fills the
-                                    GPU's CTAs best when apexes are few, e.g. 3 for the
-                                    96-atom water box; 1..64) */
-    D3_OPT_ATMB_FINE_SKIP = 14   /* block-pair kernel: 1 (default) skips out-of-range visits
-                                    per two steps, 0 per four steps (more overlap of the
-                                    packed pairs) */
+    D3_OPT_ATMB_SPLIT = 13,      /* CTAs of the precision form's block-pair kernel sharing one
+                                    apex, each taking every S-th block row (0 = automatic: the
+                                    S that fills the GPU's CTAs best when apexes are few, e.g.
+                                    3 for the 96-atom water box; 1..64). The FP64 kernels
+                                    choose theirs the same way */
+    D3_OPT_ATMB_FINE_SKIP = 14   /* precision form's block-pair kernel: 1 (default) skips
+                                    out-of-range visits per two steps, 0 per four steps (more
+                                    overlap of the packed pairs) */
 };
 int d3_set_option(d3_handle_t *handle, int option, int value);
 

@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch s
         int types = ne, tile = 0;
         for (;; --types) {
             tile = min(min(tile_max, 32 * ATM64_CHUNKS),
-                       (int)((tile_bytes - atm64_tile_fixed(NR, types)) / atm64_partner_bytes(NR, types)) & ~31);
+                       ((tile_bytes - (int)atm64_tile_fixed(NR, types)) / (int)atm64_partner_bytes(NR, types)) & ~31);
             if (types == 1 || tile >= m) break;
         }
         if (m > 0) {

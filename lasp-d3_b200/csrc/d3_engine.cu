@@ -1226,21 +1226,26 @@ struct DBuf {
     }
 };
 
-// work space whose size follows the structures: a captured graph keeps the address it was
-// captured with, so a buffer that became too small stays until the handle goes (growing by
-// at least half, all of them together take less than three times the last)
+// work space whose size follows the structures. A captured graph keeps the address it was
+// captured with, so after a capture (keep) a buffer that became too small stays until the
+// handle goes (growing by at least half, all of them together take less than three times the
+// last)
 struct KeptBuf {
     unsigned char *p = nullptr;
     size_t n = 0;
     std::vector<unsigned char *> old;
-    void ensure(size_t m) {
+    void ensure(size_t m, bool keep) {
         if (m <= n) return;
-        unsigned char *q = nullptr;
-        const size_t want = std::max(m, n + n / 2);
-        D3_CUDA(cudaMalloc(&q, want));
-        if (p) old.push_back(p);
-        p = q;
-        n = want;
+        if (p && keep) {
+            old.push_back(p);
+            m = std::max(m, n + n / 2);
+        } else if (p) {
+            cudaFree(p);
+        }
+        p = nullptr;
+        n = 0;
+        D3_CUDA(cudaMalloc(&p, m));
+        n = m;
     }
     void release() {
         for (unsigned char *q : old) cudaFree(q);
@@ -1333,6 +1338,7 @@ struct Engine {
     DBuf<float4> atmb_scratch;
     KeptBuf atm64_scratch; // k_atm64b and, behind it, k_atm64
     Atm64Plan atm64;       // of the evaluation at hand
+    bool captured = false; // some evaluation was captured
     DBuf<double> YD64;
     DBuf<long long> atm_off;
     DBuf<int2> atm_ent;
@@ -2040,11 +2046,15 @@ static Atm64Plan atm64_plan(Engine *e, cudaStream_t s, int world) {
     Atm64Plan q;
     const bool center = e->opt.atm_surrogate && e->surr.loaded;
     const long long apexes = std::max<long long>(1, ((long long)e->n + world - 1) / world);
-    const int want = e->opt.atm_ctas_per_sm;
-    q.ctas = want <= 0 ? 1 : (want >= 4 ? 4 : (want >= 2 ? 2 : 1));
-    const size_t limit = std::min<size_t>(227 * 1024, 228 * 1024 / q.ctas - 1024) - ATM64_STATIC;
-    q.fixed = atm64_fixed_bytes(e->ne, e->nref, ATM64_THREADS / 32 / q.ctas);
-    q.tile_bytes = limit - q.fixed;
+    // CTAs per SM as asked (0: one), while each has room for the sort's cells and a tile
+    const size_t least = std::max<size_t>(ATM64_CELLS * sizeof(int), atm64_tile_fixed(e->nref, 1) + 32 * atm64_partner_bytes(e->nref, 1));
+    for (q.ctas = std::max(1, std::min(e->opt.atm_ctas_per_sm, 8));; --q.ctas) {
+        const size_t limit = std::min<size_t>(227 * 1024, 228 * 1024 / q.ctas - 1024) - ATM64_STATIC;
+        q.fixed = atm64_fixed_bytes(e->ne, e->nref, ATM64_THREADS / 32 / q.ctas);
+        q.tile_bytes = limit > q.fixed ? limit - q.fixed : 0;
+        if (q.tile_bytes >= least) break;
+        if (q.ctas == 1) throw std::runtime_error("too many element types for the ATM kernel's shared memory");
+    }
     q.split = center ? 1 : apex_split(std::max<long long>(1, (long long)e->n / world), e->dev_sms * q.ctas, 32, 0.01);
     q.grid = (int)std::min<long long>((long long)e->dev_sms * q.ctas, apexes * q.split);
     q.entries = atm64_entries(e, center);
@@ -2068,13 +2078,14 @@ static Atm64Plan atm64_plan(Engine *e, cudaStream_t s, int world) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
     const bool grow = capture == cudaStreamCaptureStatusNone;
+    e->captured |= !grow;
     if (!grow && have == 0) {
         q.scratch = reinterpret_cast<unsigned char *>(e->atmb_scratch.p);
         have = e->atmb_scratch.n * sizeof(*e->atmb_scratch.p);
     }
     if (q.blocks && grow) {
         e->YD64.ensure(yd);
-        e->atm64_scratch.ensure(widest * ATM64B_ENTRY_BYTES * q.block_cap);
+        e->atm64_scratch.ensure(widest * ATM64B_ENTRY_BYTES * q.block_cap, e->captured);
     } else if (q.blocks) {
         q.block_cap = (int)std::min<size_t>(q.block_cap, have / widest / ATM64B_ENTRY_BYTES / 32 * 32);
         q.blocks = e->YD64.n >= yd && q.block_cap >= 256;
@@ -2085,7 +2096,7 @@ static Atm64Plan atm64_plan(Engine *e, cudaStream_t s, int world) {
     while (fit && q.entries > 32 && q.grid * atm64_stride(q.entries, q.split) > have) q.entries -= 32;
     q.stride = atm64_stride(q.entries, q.split);
     if (grow || q.grid * q.stride > have) {
-        e->atm64_scratch.ensure(q.grid * q.stride);
+        e->atm64_scratch.ensure(q.grid * q.stride, e->captured);
         q.scratch = e->atm64_scratch.p;
     }
     return q;
@@ -2295,7 +2306,7 @@ static void launch_atm64(Engine *e, const KP &p0, cudaStream_t s, bool center) {
         if (k == ATM64_WEIGHTED && kind[ATM64_SIMPLE]) D3_CUDA(cudaMemsetAsync(p.work, 0, sizeof(int), s));
         atm_occupancy(e, cache[k], sm, fns[k]);
         void *args[] = {(void *)&p, (void *)&scratch, &tile_bytes, &tile_max};
-        D3_CUDA(cudaLaunchKernel(fns[k], dim3(q.grid), dim3(ATM64_THREADS / q.ctas), args, sm, s));
+        D3_CUDA(cudaLaunchKernel(fns[k], dim3(q.grid), dim3(ATM64_THREADS / 32 / q.ctas * 32), args, sm, s));
     }
 }
 
