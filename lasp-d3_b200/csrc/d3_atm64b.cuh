@@ -15,7 +15,7 @@
 //
 // Against k_atm64 (two visits a triplet, 83 FP64 operations each, nearly all lanes busy):
 // one visit of 100 operations with 70 % of the lanes in range. Bound: latency of the visit's
-// chain with three warps per scheduler (10, 11, 12 warps a CTA: 177, 162, 157 ms on 8,000
+// chain with three warps per scheduler (8, 9, 10, 12 warps a CTA: 162, 153, 147, 138 ms on 8,000
 // atoms; the shared memory and 168 registers hold no more), beside it instruction issue (47 %
 // busy, an FP64 instruction counting twice) and the shared-memory pipe (59 %). Testing every
 // step just before its visit took 186 ms instead of 157.

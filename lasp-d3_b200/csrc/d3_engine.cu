@@ -1991,15 +1991,23 @@ static int apex_split(long long apexes, long long ctas, int most, double setup) 
 }
 
 // Shape of the FP64 block-pair kernel; no warps when it is not used: FP32 form, surrogate, the
-// mirror schedule chosen, or where k_atm64 is the faster one: rows of so many types that
-// fewer than eight warps fit the shared memory (k_atm64 stages them type by type), apexes so
-// few that more than four CTAs share one and repeat its sort (16 atoms: 0.38 against 0.62 ms,
-// 32 atoms 1.14 / 1.44, 48 atoms 1.47 / 1.30, 96 atoms 2.65 / 2.12) and short lists (20,000
-// atoms with 18 entries each 1.79 / 2.01 ms, 5,000 with 62 each 0.87 / 0.83).
-// Two CTAs per SM for weight-free structures, where the set-up of one apex overlaps the
-// visits of another (8,000 atoms 157 -> 154 ms, 4,000 atoms of short lists 2.93 -> 2.50 ms);
-// one for the others, whose virial carries leave room for fewer warps in halves (2,000 atoms
-// 44.2 against 46.2 ms, batch of 48 structures 98 against 108 ms).
+// mirror schedule chosen, or where k_atm64 is the faster one: apexes so few that more than
+// four CTAs share one and repeat its sort (16 atoms: 0.38 against 0.62 ms, 32 atoms 1.14 / 1.44,
+// 48 atoms 1.47 / 1.30, 96 atoms 2.65 / 2.12), short lists (20,000 atoms with 18 entries each
+// 1.79 / 2.01 ms, 5,000 with 62 each 0.87 / 0.83), and rows of so many types that the shared
+// memory holds few warps (k_atm64 stages them type by type). ATM pass by rows / by block pairs:
+//   8,000 atoms, weight-free   5 references  5 types 12 warps 153.4 / 134.0 ms
+//                              6 types 10 warps 154.3 / 150.6, 7 types 9 warps 155.2 / 163.9
+//                              7 references  4 types 12 warps 171.6 / 151.0
+//                              5 types 10 warps 172.6 / 167.4, 6 types 8 warps 173.9 / 188.8
+//   2,000 atoms, weighted      5 references  6 types 10 warps 51.2 / 47.2, 7 types 8 warps 51.9 / 53.1
+//                              7 references  5 types 9 warps 54.1 / 53.4, 6 types 7 warps 55.0 / 62.7
+// so block pairs take at least 10 warps per SM, weighted 9. Two CTAs per SM for weight-free
+// structures where they hold as many warps as one (the set-up of one apex overlaps the visits
+// of another: 2 x 6 against 12 warps 134.0 / 138.1 ms, 2 x 5 against 10 150.6 / 152.7; but 10
+// instead of 12, 4 types and 7 references, 159.0 / 151.0); one for the others, whose virial
+// carries leave room for fewer warps in halves (2,000 atoms 44.2 against 46.2 ms, batch of 48
+// structures 98 against 108 ms).
 static Atm64bShape atm64b_shape(const Engine *e, bool simple) {
     if (!e->use_atm || e->opt.precision || e->opt.atm_schedule != 0 || (e->opt.atm_surrogate && e->surr.loaded)) return {0, 1};
     if (4 * e->n < (uint64_t)e->dev_sms) return {0, 1};
@@ -2008,13 +2016,16 @@ static Atm64bShape atm64b_shape(const Engine *e, bool simple) {
         entries += 0.5 * 4.18879020478639 * e->rc_atm * e->rc_atm * e->rc_atm * e->sg[k].natoms * e->sg[k].natoms / std::fabs(e->geoms[k].volume);
     if (entries < 48.0 * (double)e->n) return {0, 1};
     const size_t per = atm64b_warp(e->ne, e->nref, simple);
-    for (int ctas = simple ? 2 : 1; ctas >= 1; --ctas) {
+    auto warps = [&](int ctas) { // per CTA
         const size_t room = std::min<size_t>(227 * 1024, 228 * 1024 / ctas - 1024) - ATM64B_STATIC - atm64b_fixed(e->ne, e->nref);
         const int w = (int)std::min<size_t>(ATM64B_WARPS / ctas, room / per);
         // (the sort's cells and entry numbers lie in the staging area)
-        if (w * ctas >= 8 && w * per >= (ATM64_CELLS + ATM64B_MCAP) * sizeof(int)) return {w, ctas};
-    }
-    return {0, 1};
+        return w * per >= (ATM64_CELLS + ATM64B_MCAP) * sizeof(int) ? w : 0;
+    };
+    const int one = warps(1);
+    if (one < (simple ? 10 : 9)) return {0, 1};
+    if (simple && 2 * warps(2) >= one) return {warps(2), 2};
+    return {one, 1};
 }
 
 // Entries that a CTA of the FP64 ATM kernels has room for: twice the mean half list of the

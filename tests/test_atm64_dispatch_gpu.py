@@ -70,6 +70,29 @@ def test_rule_of_the_block_pairs(n, density, rc_atm, mix, table, want):
     d.close()
 
 
+# rows of (2 NR + 2) doubles per type for 32 partners and warp: 10 warps fit six types of the
+# 5-reference table or five of the other (weighted structures 10 and 9)
+@pytest.mark.gpu
+@pytest.mark.parametrize("table,most", [(0, 6), (1, 5)])
+@pytest.mark.parametrize("density", [0.02, 0.1])  # weight-free and weighted
+def test_rule_of_the_warps(table, most, density):
+    elements = [1, 6, 7, 8, 29, 14, 26]
+    for types in (most, most + 1):
+        s = box(600, density, ONE)
+        s["Z"] = np.resize(elements[:types], 600)
+        rc = dict(rc=50.0, rc_cn=25.0, rc_atm=20.0)
+        d = D3(s["Z"], 600, table=table, **rc)
+        d.set_cell(s["cell"])
+        d.set_atoms(s["pos"], s["Z"])
+        assert blocks(d) == (1 if types == most else 0)
+        e, f, st = d.compute()
+        d.close()
+        r = oracle.compute(s["pos"], s["Z"], s["cell"], c6_mode=1, extended=bool(table), **rc)
+        assert abs(e - r["energy"]) <= 1e-9 * abs(r["energy"])
+        assert np.abs(f - r["forces"]).max() <= 1e-7
+        assert np.abs(st - r["stress"]).max() <= 1e-7
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("order", [(0, 1, 0), (1, 0, 1)])
 def test_both_kinds_in_one_batch(order):
