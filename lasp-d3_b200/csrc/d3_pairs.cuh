@@ -102,9 +102,9 @@ struct PairReal<true> {
 
 // One (i, j) pair of the two-body term per unit of C6: energy C6 S, dE/dCN_i = dC6 S, force
 // scalar -6 C6 T with F_i += -6 C6 T r_ij and virial += -6 C6 T r_ij (x) r_ij (the caller
-// applies the constants, and 1/2 to the energy). q8 = s8 3 r2r4_i r2r4_j, in FP32 4/3 of it
-// (pair_q8). FP32 multiplies no two inverse powers before a power of r2 is applied: r^-16
-// leaves its range beyond 300 bohr, r^-12 beyond 1,500. The FP64 form uses
+// applies the constants, and 1/2 to the energy). q8 = s8 3 r2r4_i r2r4_j. The FP32 form
+// multiplies no two inverse powers before a power of r2 is applied: r^-16 leaves its range
+// beyond 300 bohr, r^-12 beyond 1,500. The FP64 form uses
 // reciprocals and roots refined by one third-order step instead of divisions: 11 FP64
 // operations for S and T (Becke-Johnson) where four IEEE divisions took over 60.
 template <typename R>
@@ -115,24 +115,17 @@ __device__ __forceinline__ R pair_rcp(R x) {
         return rcp_nr(x);
 }
 template <typename R>
-__device__ __forceinline__ R pair_q8(double q) {
-    return (R)(sizeof(R) == 4 ? q * (4.0 / 3.0) : q);
-}
-template <typename R>
 __device__ __forceinline__ void pair_term(const KP &p, R r2, R A6_or_R0, R A8, R q8, R &S, R &T) {
-    constexpr bool F32 = sizeof(R) == 4;
     const R s6 = (R)p.s6;
     if (p.damping == 1) {
         const R r4 = r2 * r2;
         const R i6 = pair_rcp<R>(fma(r4, r2, A6_or_R0)), i8 = pair_rcp<R>(fma(r4, r4, A8));
         const R x6 = s6 * i6, x8 = q8 * i8;
-        if constexpr (F32) {
-            S = fma(0.75f, x8, x6);
-            T = fma(x8 * r2, r4 * i8, x6 * (r4 * i6));
-        } else {
-            S = x6 + x8;
+        S = x6 + x8;
+        if constexpr (sizeof(R) == 4)
+            T = fma(4.0f / 3.0f * x8 * r2, r4 * i8, x6 * (r4 * i6));
+        else
             T = r4 * fma((R)(4.0 / 3.0) * x8 * i8, r2, x6 * i6);
-        }
     } else {
         R ir;
         if constexpr (sizeof(R) == 4)
@@ -146,8 +139,8 @@ __device__ __forceinline__ void pair_term(const KP &p, R r2, R A6_or_R0, R A8, R
         const R f6 = pair_rcp<R>(fma((R)6 * x6_14, (R)1, (R)1)), f8 = pair_rcp<R>(fma((R)6 * x8_8, x8_8, (R)1));
         // f6' = 14 x6^14 f6 = 7/3 (1 - f6), f8' = 12 x8^16 f8 = 2 (1 - f8)
         const R y6 = s6 * f6 * ir6, y8 = q8 * f8 * ir8;
-        S = F32 ? fma((R)0.75, y8, y6) : y6 + y8;
-        T = ir2 * (y6 * fma((R)(-7.0 / 3.0), (R)1 - f6, (R)1) + (F32 ? y8 : (R)(4.0 / 3.0) * y8) * fma((R)-2, (R)1 - f8, (R)1));
+        S = y6 + y8;
+        T = ir2 * (y6 * fma((R)(-7.0 / 3.0), (R)1 - f6, (R)1) + (R)(4.0 / 3.0) * y8 * fma((R)-2, (R)1 - f8, (R)1));
     }
 }
 
@@ -252,13 +245,13 @@ __global__ void __launch_bounds__(PAIRS_WARPS * 32, 2) k_twobody_g(KP p, int *wo
     extern __shared__ __align__(16) unsigned char smp[];
     const int ne = p.ne;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // per type pair: BJ A^6, A^8 (zero damping: R0) and q8
+    // per type pair: BJ A^6, A^8 (zero damping: R0) and s8 3 r2r4_i r2r4_j
     R *ptab = reinterpret_cast<R *>(smp);
     for (int k = threadIdx.x; k < ne * ne; k += blockDim.x) {
         const double *pa = p.pairA + (size_t)k * 4;
         ptab[3 * k] = (R)pa[0];
         ptab[3 * k + 1] = (R)pa[1];
-        ptab[3 * k + 2] = pair_q8<R>(p.s8 * 3.0 * p.r2r4[k / ne] * p.r2r4[k % ne]);
+        ptab[3 * k + 2] = (R)(p.s8 * 3.0 * p.r2r4[k / ne] * p.r2r4[k % ne]);
     }
     __syncthreads();
     const size_t tab_bytes = ((size_t)3 * ne * ne * sizeof(R) + 15) & ~(size_t)15;
