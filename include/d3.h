@@ -130,10 +130,9 @@ enum {
                                     and leaves the ATM terms out instead */
     D3_OPT_PAIR_KERNEL = 10,     /* two-body pass: 0 (default) compact groups of 32 atoms with
                                     staged partners (one thread per atom); 1 one warp per atom
-                                    (also used for sharded evaluations and handles of more
-                                    than 8 elements) */
+                                    (also used for handles of more than 8 elements) */
     D3_OPT_ATMB_WARPS = 11,      /* precision-form block-pair ATM kernel: warps per CTA, 0 =
-                                    automatic (8), 2..12; above 8 each warp stages one y
+                                    automatic (up to 12), 2..12; above 8 each warp stages one y
                                     block at a time instead of two. With
                                     D3_OPT_ATM_CTAS_PER_SM = 2, two CTAs per SM when they fit */
     D3_OPT_ATMB_LIST_CAPACITY = 12, /* longest half list (entries) the precision form's
@@ -212,8 +211,8 @@ int d3_launches_per_eval(d3_handle_t *handle);
 
 /* Self-check of the refined reciprocal square root, reciprocal and inverse cube
    root used by the ATM kernel: max relative error against CUDA's double-precision
-   functions over [1e-12, 1e14], written to max_rel_err[6] (one Newton step:
-   rsqrt, rcp, rcbrt; two Newton steps: rsqrt, rcp, rcbrt). */
+   functions over [1e-12, 1e14], written to max_rel_err[6] (one step, of third order for
+   rsqrt and rcp: rsqrt, rcp, rcbrt; a further Newton step: rsqrt, rcp, rcbrt). */
 int d3_selftest_math(double *max_rel_err);
 
 /* Measured FMA throughput (TFLOP/s, 2 flops per FMA) of the FP64 (fp64 = 1) or FP32

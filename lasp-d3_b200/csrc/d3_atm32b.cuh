@@ -1,7 +1,7 @@
 // ATM three-body kernel, precision form, block-pair schedule: every triplet visited once.
 // Included by d3_engine.cu after k_atm32 (same per-entry set-up, weights and outputs).
 //
-// Per apex a (persistent CTAs take apexes from a work counter, largest lists first):
+// Per apex a (persistent CTAs take apexes from a work counter):
 //  1. The entries of the half list are counting-sorted by the Hilbert-curve position of their
 //     cell in a 16^3 grid over [-rc, rc]^3 around the apex, so 32 consecutive entries ("a
 //     block") are close in space.

@@ -1927,9 +1927,8 @@ static AtmbShape blockpair_shape(const Engine *e) {
 }
 static int blockpair_warps(const Engine *e) { return blockpair_shape(e).warps; }
 
-// the two-body pass on atom groups (d3_pairs.cuh), unless chosen off or the handle has more
-// element types than the staged rows hold; sharded evaluations (which split by central
-// atom) take the per-atom kernels whatever this says
+// the pair passes on atom groups (d3_pairs.cuh), unless chosen off or the handle has more
+// element types than the staged rows hold (sharded evaluations too: a rank takes whole groups)
 static bool pairs_grouped(const Engine *e) { return e->opt.pair_kernel == 0 && e->ne <= PAIRS_MAX_TYPES; }
 
 static size_t pairs_smem(const Engine *e) {
@@ -1976,7 +1975,7 @@ static int pairs_occupancy(Engine *e) {
 // CTAs that share one apex (systems of few apexes): apexes are equally long, so a pass takes
 // ceil(apexes S / CTAs) waves of items, each an S-th of an apex and the set-up that every
 // split repeats (`setup`, in apexes). The S of the shortest pass; without it 16 and 96 apexes
-// leave most of the 148 SMs idle (FP64 ATM pass 26.8 and 36 ms, with it 0.4 and 3.3 ms).
+// leave most of the 148 SMs idle (FP64 ATM pass of 16 atoms 0.37 ms with it, of 96 atoms 2.3).
 static int apex_split(long long apexes, long long ctas, int most, double setup) {
     int best = 1;
     double least = 1e300;
@@ -2789,7 +2788,7 @@ int engine_launches_per_eval(const Engine *e) {
     return (blocks ? 17 : 16) + pairs;
 }
 
-// Accuracy check of the Newton-refined helpers used by the ATM kernel against CUDA's
+// Accuracy check of the refined roots (d3_roots.cuh) of the pair and ATM kernels against CUDA's
 // double-precision 1/sqrt, 1/x and cbrt over log-spaced inputs in [1e-12, 1e14].
 __global__ void k_selftest_math(double *err, int m) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
