@@ -93,10 +93,10 @@ struct Atm64X {
     Atm64Row e;
     double w[MAX_NREF + 1], dw[MAX_NREF + 1];
 };
-// scratch of one CTA: the entries set up at once, then the rows of its split by type
+// scratch of one CTA: the rows of its split by type, then the entries set up at once
 struct Atm64Scratch {
     unsigned char *p;
-    size_t stride; // bytes per CTA
+    unsigned int stride, first; // bytes per CTA, of its rows
     int entries;
 };
 
@@ -309,10 +309,18 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch s
     unsigned short *list = reinterpret_cast<unsigned short *>(queue + 8 * ATM64_QCAP);             // [ATM64_LIST]
     unsigned char *area = sm64 + atm64_fixed_bytes(ne, NR, nw);
     int *cells = reinterpret_cast<int *>(area); // [ATM64_CELLS] while the entries are sorted
+    // (the entries' address and number, needed between the visits only, are read from shared
+    // memory there: in registers they made 2,000 atoms of 12 types and 7 references 1 % slower)
+    __shared__ Atm64Row *volatile s_entries;
+    __shared__ volatile int s_ecap;
     __shared__ int s_item, s_row, s_tot[ATM64_THREADS / 32];
     __shared__ double red[ATM64_THREADS / 32][11], s_sums[ATM64_THREADS / 32][ATM64_SR], s_coef[16][4];
     __shared__ unsigned long long s_rule[16];
     double *sr = s_sums[warp];
+    if (tid == 0) {
+        s_entries = reinterpret_cast<Atm64Row *>(scratch.p + (size_t)blockIdx.x * scratch.stride + scratch.first);
+        s_ecap = scratch.entries;
+    }
     if (tid < 16) atm64_rules(KIND == ATM64_WEIGHTED, tid, s_rule[tid], s_coef[tid]);
     if (lane == 0) {
         sr[ATM64_S1] = 1.0;
@@ -320,9 +328,7 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch s
     }
     if (warp_uniform(p.atm_off[p.n] > p.atm_cap ? 1 : 0)) return; // list overflowed: the host grows it and re-runs
     for (int k = tid; k < ne * ne; k += blockDim.x) r0sq[k] = p.r0ab[k] * p.r0ab[k];
-    const int ecap = scratch.entries;
-    Atm64Row *entries = reinterpret_cast<Atm64Row *>(scratch.p + blockIdx.x * scratch.stride);
-    Atm64X *rows = reinterpret_cast<Atm64X *>(entries + ecap);
+    Atm64X *rows = reinterpret_cast<Atm64X *>(scratch.p + (size_t)blockIdx.x * scratch.stride);
     const double third = 1.0 / 3.0;
     const double rc = sqrt(p.ratm2), cinv = 16.0 / (2.0 * rc);
     // FP32 range test: |d3 - half| <= half in range, but near either end of [0, 2 half] the
@@ -356,7 +362,7 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch s
         int types = ne, tile = 0;
         for (;; --types) {
             tile = min(min(tile_max, 32 * ATM64_CHUNKS),
-                       ((tile_bytes - (int)atm64_tile_fixed(NR, types)) / (int)atm64_partner_bytes(NR, types)) & ~31);
+                       (int)(((unsigned)tile_bytes - (unsigned)atm64_tile_fixed(NR, types)) / (unsigned)atm64_partner_bytes(NR, types)) & ~31);
             if (types == 1 || tile >= m) break;
         }
         if (m > 0) {
@@ -368,10 +374,11 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch s
         float4 *sC = sF + tile + 32;                                  // [ATM64_CHUNKS][2]: box of each chunk, sphere radius
         double2 *sR = reinterpret_cast<double2 *>(sC + 2 * ATM64_CHUNKS); // [types][tile + 1][RQ]
         double acc = 0; // this lane's apex sum (lanes 0..10: energy, dE/dCN, force, virial)
-        for (int b0 = 0; b0 < m; b0 += ecap) {
+        for (int b0 = 0; b0 < m; b0 += s_ecap) {
             // set up the entries in Hilbert order (counting sort on a 16^3, 8^3 or 4^3 grid,
             // whose curves are prefixes of one another) and list this split's rows by type
-            const int bn = min(ecap, m - b0);
+            const int bn = min(s_ecap, m - b0);
+            Atm64Row *entries = s_entries;
             const int hs = bn >= 1024 ? 0 : (bn >= 128 ? 3 : 6), ncell = ATM64_CELLS >> hs;
             auto cell_of = [&](const int2 ent) {
                 const double3 v = atm64_pos(p, g, xa, ent, p.xs[ent.x]);
@@ -421,10 +428,11 @@ __global__ void __launch_bounds__(ATM64_THREADS, 1) k_atm64(KP p, Atm64Scratch s
                     const int r0 = warp_uniform(toff[t0]), r1 = warp_uniform(toff[t0 + tn]);
                     if (r0 == r1 && t0 != 0) continue;
                     if (tid == 0) s_row = r0;
+                    const Atm64Row *staged = s_entries;
                     for (int k = tid; k < cnt; k += blockDim.x) {
                         int j, tj;
-                        if (m <= ecap) {
-                            const Atm64Row *src = entries + p0 + k;
+                        if (m <= s_ecap) {
+                            const Atm64Row *src = staged + p0 + k;
                             j = src->j;
                             tj = src->t;
                             if (t0 == 0) {

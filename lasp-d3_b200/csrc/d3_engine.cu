@@ -2028,8 +2028,10 @@ static Atm64bShape atm64b_shape(const Engine *e, bool simple) {
 }
 
 // Entries that a CTA of the FP64 ATM kernels has room for: twice the mean half list of the
-// densest structure (slabs and clusters in vacuum; centre mode: full lists) and some, at most
-// what the images within rc_ATM allow. Longer lists are right too, k_atm64 takes them in parts.
+// densest structure and some (slabs and clusters in vacuum; centre mode: full lists), at least
+// 2,048 as far as the images within rc_ATM allow, in weight-free structures every other atom.
+// Longer lists are right too, k_atm64 takes them in parts (a cluster of 1,500 atoms with room
+// for 1,024: ATM pass 5.2 ms instead of 4.6).
 static int atm64_entries(const Engine *e, bool center) {
     double most = 0.0;
     for (size_t k = 0; k < e->sg.size(); ++k) {
@@ -2037,7 +2039,7 @@ static int atm64_entries(const Engine *e, bool center) {
         const double mean = (center ? 1.0 : 0.5) * 4.18879020478639 * e->rc_atm * e->rc_atm * e->rc_atm * q.natoms / std::fabs(e->geoms[k].volume);
         double images = q.natoms;
         for (int i = 0; i < 3; ++i) images *= std::floor(2.0 * q.ratm_frac[i]) + 1.0;
-        most = std::max(most, std::min(images, std::max(1024.0, 2.0 * mean + 256.0)));
+        most = std::max(most, q.atm_simple ? images : std::min(images, std::max(2048.0, 2.0 * mean + 256.0)));
     }
     return (int)(std::ceil(std::min(most, (double)ATM64_ENTRIES) / 256.0) * 256.0);
 }
@@ -2056,7 +2058,10 @@ static Atm64Plan atm64_plan(Engine *e, cudaStream_t s, int world) {
     Atm64Plan q;
     const bool center = e->opt.atm_surrogate && e->surr.loaded;
     const long long apexes = std::max<long long>(1, ((long long)e->n + world - 1) / world);
-    // CTAs per SM as asked (0: one), while each has room for the sort's cells and a tile
+    // CTAs per SM as asked (0: one), while each has room for the sort's cells and a tile (and
+    // so for what k_atm64 subtracts from the tile area at any number of types)
+    static_assert(atm64_tile_fixed(5, MAX_TYPES) <= ATM64_CELLS * sizeof(int) && atm64_tile_fixed(7, MAX_TYPES) <= ATM64_CELLS * sizeof(int),
+                  "fixed part of the tile area");
     const size_t least = std::max<size_t>(ATM64_CELLS * sizeof(int), atm64_tile_fixed(e->nref, 1) + 32 * atm64_partner_bytes(e->nref, 1));
     for (q.ctas = std::max(1, std::min(e->opt.atm_ctas_per_sm, 8));; --q.ctas) {
         const size_t limit = std::min<size_t>(227 * 1024, 228 * 1024 / q.ctas - 1024) - ATM64_STATIC;
@@ -2309,7 +2314,7 @@ static void launch_atm64(Engine *e, const KP &p0, cudaStream_t s, bool center) {
     const size_t sm = q.fixed + q.tile_bytes;
     int tile_bytes = (int)q.tile_bytes;
     int tile_max = e->opt.atm_tile > 0 ? std::max(32, std::min(e->opt.atm_tile, 65504) & ~31) : 65504;
-    Atm64Scratch scratch{q.scratch, q.stride, q.entries};
+    Atm64Scratch scratch{q.scratch, (unsigned int)q.stride, (unsigned int)(q.stride - q.entries * sizeof(Atm64Row)), q.entries};
     p.atmb_split = q.split;
     for (int k = 0; k < 3; ++k) {
         if (!kind[k]) continue;

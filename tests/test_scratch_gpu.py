@@ -102,3 +102,22 @@ def test_capture_right_after_a_change_of_form():
     assert abs(e - e1) <= 1e-11 * abs(e1) and np.abs(f - f1).max() <= 1e-9
     ref.close()
     d.close()
+
+
+@pytest.mark.parametrize("n,pad", [(1500, 30.0), (300, 20.0)])
+def test_lists_longer_than_the_room_for_them(n, pad):
+    """Clusters in vacuum, whose lists are many times the mean that the room is sized by (weighted
+    and weight-free cells): by block pairs or rows, whole or in parts, as the FP64 oracle."""
+    import oracle
+
+    s = box(n, 0.1)
+    edge = float(s["cell"][0, 0]) + pad
+    s = dict(s, cell=np.eye(3) * edge)
+    rc = dict(rc=45.0, rc_cn=25.0, rc_atm=40.0)
+    d = handle(s, **rc)
+    e, f, st = d.compute()
+    d.close()
+    r = oracle.compute(s["pos"], s["Z"], s["cell"], c6_mode=1, **rc)
+    assert abs(e - r["energy"]) <= 1e-9 * abs(r["energy"])
+    assert np.abs(f - r["forces"]).max() <= 1e-7
+    assert np.abs(st - r["stress"]).max() <= 1e-7
