@@ -1348,7 +1348,7 @@ struct Engine {
     // ([0] group count, [1] work items taken), per-slice partial sums, per-structure flags
     std::vector<int4> srow_host;
     DBuf<int4> srows, groups;
-    DBuf<int> gctl, anyshift;
+    DBuf<int> gctl;
     DBuf<double> gpart;
     size_t group_bound = 0;
     DBuf<double> out;
@@ -1402,7 +1402,6 @@ struct Engine {
         srows.release();
         groups.release();
         gctl.release();
-        anyshift.release();
         gpart.release();
         sg_dev.release();
         status.release();
@@ -1611,14 +1610,13 @@ Engine *engine_create(const uint16_t *elements, uint64_t n_elements, uint64_t ma
         e->G.ensure(N);
         e->atm_cnt.ensure(N);
         e->atm_off.ensure(N + 1);
-        e->work.ensure(1);
+        e->work.ensure(1 + 7 * max_structs); // work counter; per structure a flag, then the six extents
         e->sid_in.ensure(N);
         e->sid.ensure(N);
         e->sg_dev.ensure(max_structs);
         e->out.ensure(10 * max_structs + 3 * N);
         e->status.ensure(1);
         e->counters.ensure(4);
-        e->anyshift.ensure(7 * max_structs); // flag, then the six extents, per structure
         for (auto &x : e->ev) D3_CUDA(cudaEventCreate(&x));
         e->host_out.resize(10 * max_structs + 3 * N);
         return e;
@@ -2179,8 +2177,8 @@ static KP make_kp(Engine *e, cudaStream_t s, int rank = 0, int world = 1) {
         if (e->atm64.blocks) p.YD64 = e->YD64.p;
     }
     p.atm_force_scaled = e->opt.atm_force_scaled ? 1 : 0;
-    p.anyshift = e->anyshift.p;
-    p.span = reinterpret_cast<unsigned int *>(e->anyshift.p + e->nstruct);
+    p.anyshift = e->work.p + 1;
+    p.span = reinterpret_cast<unsigned int *>(p.anyshift + e->nstruct);
     p.srows = e->srows.p;
     p.nsrow = (int)e->srow_host.size();
     p.groups = e->groups.p;
@@ -2545,7 +2543,7 @@ static KP eval_lists(Engine *e, EvalLists &r, bool ref_order, cudaStream_t s) {
     p.atm_ref_order = ref_order ? 1 : 0;
     p.counters = nullptr;
     p.nstruct = (int)e->sg.size();
-    p.span = reinterpret_cast<unsigned int *>(e->anyshift.p + e->sg.size());
+    p.span = reinterpret_cast<unsigned int *>(p.anyshift + e->sg.size());
     p.sg = r.sg.p;
     p.stencils = r.rows.p;
     p.bin_start = r.bins.p + nbins;
